@@ -41,7 +41,12 @@ mv_tuning_entry tuned_params(int dim, int64_t n);
 // mv_staged.cu
 cudaError_t launch_stage(int kernel, const Job& J, const StageJob& SJ, const JobTable& TB, int blocks,
                          cudaStream_t st);
-int stage_blocks_per_sm(int kernel, int precision);
+int stage_blocks_per_sm(int kernel);
+// mv_clip.cu
+cudaError_t launch_clip(const Job& J, const StageJob& SJ, const JobTable& TB, bool wide, int resident,
+                        cudaStream_t st);
+int clip_blocks_per_sm(int precision, bool wide);
+// mv_staged.cu
 int stage_list_stride();
 int stage_wide_stride();
 cudaError_t launch_append_range(int32_t* dst, int32_t first, int32_t count, cudaStream_t st);
@@ -214,7 +219,7 @@ struct mv_context {
   int sm_count = 0;
   int bps_fast[2] = {0, 0};
   int bps_large[2] = {0, 0};
-  int bps_stage[4][2] = {};  // shell, clip, integral, wide-shell kernels by precision
+  int bps_stage[5][2] = {};  // shell, clip, integral, wide-shell, wide-clip kernels by precision
   std::vector<cudaEvent_t> stage_ev;  // 4 per chunk: before shell, clip, integral, after
   double rec_words_hint = 0.0;  // record words per cell the last staged build needed
   Workspace ws;
@@ -338,6 +343,16 @@ bool use_staged(const mv_options& o, int64_t n, int dim) {
 
 int64_t record_words_per_cell(int dim) { return dim == 3 ? 352 : (dim == 2 ? 224 : 128); }
 
+// One stage kernel (0 shell, 1 clip, 2 integrals, 3 wide shell, 4 wide clip) over SJ's
+// cells: the resident grid, or fewer blocks when those give every cell a warp (the clip
+// kernel: a group of lanes) already.
+cudaError_t run_stage_kernel(const mv_context* ctx, int kernel, const Job& J, const StageJob& SJ,
+                             const JobTable& TB, int pi, cudaStream_t st) {
+  const int resident = ctx->sm_count * std::max(1, ctx->bps_stage[kernel][pi]);
+  if (kernel == 1 || kernel == 4) return launch_clip(J, SJ, TB, kernel == 4, resident, st);
+  return launch_stage(kernel, J, SJ, TB, std::max(1, std::min(resident, (SJ.nitems + 3) / 4)), st);
+}
+
 // Shell, clip and integral kernels over chunks of cells in processing (grid) order.
 // Cells the first shell does not decide are appended to the retry list; *n_retry
 // receives their number.
@@ -418,13 +433,9 @@ int run_staged(mv_context* ctx, const Job& J, const JobTable& TB, int dim, const
     SJ.work = reinterpret_cast<unsigned int*>(ctr + 1 + 3 * c);
     SJ.rec_counter = keep_records ? keep_records : ctr + 1 + 3 * c + 2;
     SJ.box = ((probe && c == 0) || box_mode) ? 1 : 0;
-    const int64_t warps_needed = SJ.nitems;
     for (int k = 0; k < 3; k++) {
-      const int wpb = 4;  // every stage kernel runs 4 warps per block
-      int64_t blocks = (int64_t)ctx->sm_count * std::max(1, ctx->bps_stage[k][pi]);
-      blocks = std::min<int64_t>(blocks, (warps_needed + wpb - 1) / wpb);
       MV_CUDA(cudaEventRecord(ctx->stage_ev[4 * c + k], st));
-      MV_CUDA(launch_stage(k, J, SJ, TB, (int)std::max<int64_t>(1, blocks), st));
+      MV_CUDA(run_stage_kernel(ctx, k, J, SJ, TB, pi, st));
       (*launches)++;
     }
     MV_CUDA(cudaEventRecord(ctx->stage_ev[4 * c + 3], st));
@@ -494,12 +505,10 @@ int run_staged(mv_context* ctx, const Job& J, const JobTable& TB, int dim, const
       SW.nitems = (int32_t)std::min<int64_t>(chunk2, nr - c * chunk2);
       SW.work = reinterpret_cast<unsigned int*>(ctr + ctr2 + 1 + 3 * c);
       SW.rec_counter = ctr + ctr2 + 1 + 3 * c + 2;
-      const int kern[3] = {3, 1, 2};
+      const int kern[3] = {3, 4, 2};
       for (int k = 0; k < 3; k++) {
-        int64_t blocks = (int64_t)ctx->sm_count * std::max(1, ctx->bps_stage[kern[k]][pi]);
-        blocks = std::min<int64_t>(blocks, (SW.nitems + 3) / 4);
         MV_CUDA(cudaEventRecord(ctx->stage_ev[4 * c + k], st));
-        MV_CUDA(launch_stage(kern[k], J, SW, TB, (int)std::max<int64_t>(1, blocks), st));
+        MV_CUDA(run_stage_kernel(ctx, kern[k], J, SW, TB, pi, st));
         (*launches)++;
       }
       MV_CUDA(cudaEventRecord(ctx->stage_ev[4 * c + 3], st));
@@ -1749,7 +1758,8 @@ int mv_context_create(int device, mv_context** out) {
   for (int p = 0; p < 2; p++) {
     ctx->bps_fast[p] = cells_blocks_per_sm_fast(p);
     ctx->bps_large[p] = cells_blocks_per_sm_large(p);
-    for (int k = 0; k < 4; k++) ctx->bps_stage[k][p] = stage_blocks_per_sm(k, p);
+    for (int k = 0; k < 5; k++)
+      ctx->bps_stage[k][p] = k == 1 || k == 4 ? clip_blocks_per_sm(p, k == 4) : stage_blocks_per_sm(k);
   }
   if (cudaGetLastError() != cudaSuccess || ctx->bps_fast[0] <= 0 || ctx->bps_fast[1] <= 0) {
     cudaStreamDestroy(ctx->stream);

@@ -59,12 +59,6 @@ __device__ __forceinline__ int warp_excl_scan(int v, int lane, int* total) {
   return x - v;
 }
 
-__device__ __forceinline__ double warp_max(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(FULL, v, o));
-  return v;
-}
-
 // Largest non-negative double over the warp: non-negative binary64 values order like
 // their bit patterns, so two 32-bit warp reductions give the exact maximum.
 __device__ __forceinline__ double warp_max_nonneg(double v) {
@@ -73,10 +67,6 @@ __device__ __forceinline__ double warp_max_nonneg(double v) {
   const unsigned mhi = __reduce_max_sync(FULL, hi);
   const unsigned mlo = __reduce_max_sync(FULL, hi == mhi ? lo : 0u);
   return __longlong_as_double((long long)(((unsigned long long)mhi << 32) | mlo));
-}
-
-__device__ __forceinline__ D3 shfl_d3(D3 v, int src) {
-  return {__shfl_sync(FULL, v.x, src), __shfl_sync(FULL, v.y, src), __shfl_sync(FULL, v.z, src)};
 }
 
 template <int NW>
@@ -102,13 +92,6 @@ __device__ __forceinline__ int select_bit(const unsigned (&m)[NW], int s) {
     s -= c;
   }
   return -1;
-}
-
-// position of the s-th (1-based) set bit of a 64-bit mask
-__device__ __forceinline__ int select64(unsigned long long m, int s) {
-  const unsigned lo = (unsigned)m;
-  const int c = __popc(lo);
-  return s <= c ? (int)__fns(lo, 0, s) : 32 + (int)__fns((unsigned)(m >> 32), 0, s - c);
 }
 
 __device__ __forceinline__ unsigned valid_bits(int nv, int w) {
@@ -158,24 +141,9 @@ __device__ __noinline__ int exact_clip(const Job& J, const SM& S, int s, D3 x, D
   return in_sphere_exact_sign(A, B, C, Dd, W);
 }
 
-// Whether the exact decision of exact_clip is the zero determinant of five corners of
-// one axis-aligned box (box_corners), found without multi-limb arithmetic: the vertex
-// is then kept.
-template <class SM>
-__device__ __noinline__ bool exact_clip_box_zero(const Job& J, const SM& S, int s, D3 x, D3 ngb) {
-  int64_t A[3], B[3], C[3], Dd[3], W[3];
-  iloc(J, x, A);
-  iloc(J, right_loc(J, S, S.vd0[s], x), B);
-  iloc(J, right_loc(J, S, S.vd1[s], x), C);
-  iloc(J, right_loc(J, S, S.vd2[s], x), Dd);
-  iloc(J, ngb, W);
-  return box_corners(A, B, C, Dd, W);
-}
-
 // Vertex::from_dual (convex_cell.rs:28-48) into slot `slot`; *r2 receives the
-// vertex's squared distance to the generator (kept in S.vr2 when STORE_R2; otherwise
-// vertex_r2 recomputes it).
-template <class PIdx, bool STORE_R2 = true, class SM>
+// vertex's squared distance to the generator.
+template <class PIdx, class SM>
 __device__ __forceinline__ bool make_vertex(SM& S, int slot, int i, int j, int k, D3 x, int dim,
                                             double* r2) {
   D3 loc;
@@ -190,7 +158,7 @@ __device__ __forceinline__ bool make_vertex(SM& S, int slot, int i, int j, int k
   S.vx[slot] = loc.x;
   S.vy[slot] = loc.y;
   S.vz[slot] = loc.z;
-  if constexpr (STORE_R2) S.vr2[slot] = rr;
+  S.vr2[slot] = rr;
   S.f4[slot] = make_float4(__double2float_rn(loc.x - x.x), __double2float_rn(loc.y - x.y),
                            __double2float_rn(loc.z - x.z), 0.f);
   S.vd0[slot] = (PIdx)i;
@@ -198,17 +166,6 @@ __device__ __forceinline__ bool make_vertex(SM& S, int slot, int i, int j, int k
   S.vd2[slot] = (PIdx)k;
   *r2 = rr;
   return true;
-}
-
-// The squared distance of the vertex in slot `slot` to the generator, as make_vertex
-// computes it (Vertex::from_dual, convex_cell.rs:38-42).
-template <class SM>
-__device__ __forceinline__ double vertex_r2(const SM& S, int slot, D3 x, int dim) {
-  D3 dl = {S.vx[slot], S.vy[slot], S.vz[slot]};
-  if (dim == 1) dl = {dl.x, 0.0, 0.0};
-  if (dim == 2) dl = {dl.x, dl.y, 0.0};
-  const D3 r = sub(x, dl);
-  return dot(r, r);
 }
 
 // Vertex duals of the initial cuboid (convex_cell.rs:298-307), one vertex per lane.
@@ -229,15 +186,6 @@ __device__ __forceinline__ void cuboid_duals(int lane, int* i0, int* i1, int* i2
 // extruded dimensions, whose vertex coordinates are +-0.5.
 __device__ __forceinline__ double amax_of(double max_r2, int dim) {
   return sqrt((max_r2 + 0.26 * (3 - dim)) * (1.0 + 1e-9)) * (1.0 + 1e-9);
-}
-
-// The same bound in f32, rounded up, from the safety radius sr = 2 sqrt(max_r2):
-// sqrt(max_r2) <= sr / 2 (1 + 2^-52), |v - x| exceeds the rounded sqrt(max_r2) by a
-// few ulps at most, and sqrt(a + b) <= sqrt(a) + sqrt(b) covers the extruded
-// dimensions (sqrt(0.26) < 0.51, sqrt(0.52) < 0.7212).
-__device__ __forceinline__ float amax32_of_sr(double sr, int dim) {
-  const float h = __fmul_ru(__double2float_ru(sr), 0.50000006f);
-  return dim == 3 ? h : __fadd_ru(h, dim == 2 ? 0.51f : 0.7212f);
 }
 
 enum CellResult {
@@ -967,92 +915,6 @@ __device__ __noinline__ int ring_replay_warp(SM& S, int lane, int nvf, int nv, i
   return len;
 }
 
-// ring_replay_warp for at most 32 removed vertices with each triangle held by its lane:
-// lane j starts with the triangle at position nvf + j and tracks the position the
-// reference's swaps give it (the triangle at position i moves to the winner's position
-// when step i takes a later one), so a step is a reduction of the positions of the
-// triangles that extend the cycle rather than a scan of shared memory.  The removed
-// vertices' order in `ord` is left as it was: only their slots are reused, and the
-// vertices that replace them take ring order.  Returns as ring_replay_warp.
-template <class T, class SM>
-__device__ __noinline__ int ring_replay_lanes(SM& S, int lane, int nvf, int nv, int np) {
-  using PIdx = typename T::PIdx;
-  const int n = nv - nvf;
-  if (n > 32) return ring_replay_warp<T>(S, lane, nvf, nv, np);
-  for (int i = lane; i < np; i += 32) S.rptr[i] = (PIdx)i;
-  int t[3] = {0, 0, 0};
-  if (lane < n) {
-    const int sl = S.ord[nvf + lane];
-    t[0] = S.vd0[sl], t[1] = S.vd1[sl], t[2] = S.vd2[sl];
-  }
-  int pos = lane;
-  bool open = lane > 0 && lane < n;  // not yet part of the cycle
-  int start = __shfl_sync(FULL, t[0], 0);
-  __syncwarp();
-  if (lane == 0) {
-    S.rptr[t[0]] = (PIdx)t[1];
-    S.rptr[t[1]] = (PIdx)t[2];
-    S.rptr[t[2]] = (PIdx)t[0];
-  }
-  __syncwarp();
-  int len = 3;
-  for (int i = 1; i < n; i++) {
-    int code = 0;  // 1 + 2 * rotation + case (0: grow the cycle, 1: absorb a node)
-    if (open) {
-      const bool in[3] = {S.rptr[t[0]] != (PIdx)t[0], S.rptr[t[1]] != (PIdx)t[1],
-                          S.rptr[t[2]] != (PIdx)t[2]};
-#pragma unroll
-      for (int a = 0; a < 3; a++) {
-        const int j = a == 2 ? 0 : a + 1, k = a == 0 ? 2 : a - 1;
-        if (code == 0) {
-          if (!in[a] && in[j] && in[k] && S.rptr[t[k]] == (PIdx)t[j])
-            code = 1 + 2 * a;
-          else if (in[a] && in[j] && in[k] && S.rptr[t[k]] == (PIdx)t[j] && S.rptr[t[j]] == (PIdx)t[a])
-            code = 2 + 2 * a;
-        }
-      }
-    }
-    const unsigned key = code ? (unsigned)pos : 64u;
-    const unsigned m = __reduce_min_sync(FULL, key);
-    if (m == 64u) return -1;
-    const int w = __ffs(__ballot_sync(FULL, key == m)) - 1;
-    const int how = __shfl_sync(FULL, code, w);
-    const int a = (how - 1) >> 1;
-    const int w0 = __shfl_sync(FULL, t[0], w), w1 = __shfl_sync(FULL, t[1], w),
-              w2 = __shfl_sync(FULL, t[2], w);
-    const int ta = a == 0 ? w0 : (a == 1 ? w1 : w2);
-    const int tb = a == 0 ? w1 : (a == 1 ? w2 : w0);
-    const int tc = a == 0 ? w2 : (a == 1 ? w0 : w1);
-    const bool grow = ((how - 1) & 1) == 0;
-    __syncwarp();
-    if (lane == 0) {
-      S.rptr[tc] = (PIdx)ta;
-      S.rptr[grow ? ta : tb] = (PIdx)tb;
-    }
-    if (lane == w) open = false;
-    else if (open && pos == i) pos = (int)m;  // swap(i, m) of compute_boundary
-    if (grow) {
-      len += 1;
-    } else {
-      if (start == tb) start = ta;
-      len -= 1;
-    }
-    __syncwarp();
-  }
-  if (len > T::VMAX) return -2;
-  if (lane == 0) {
-    int cur = start;
-    for (int e = 0; e < len; e++) {
-      const int nxt = S.rptr[cur];
-      S.ea[e] = (PIdx)cur;
-      S.eb[e] = (PIdx)nxt;
-      cur = nxt;
-    }
-  }
-  __syncwarp();
-  return len;
-}
-
 // Parallel ring: the boundary edges of the union of the removed dual triangles form
 // the same cycle the serial algorithm builds; it starts at the first removed
 // vertex's dual[0] whenever that node is still on the boundary.  Returns the edge
@@ -1114,94 +976,14 @@ __device__ __forceinline__ int ring_parallel(SM& S, int lane, int nvf, int nv) {
   return ok ? E : -1;
 }
 
-// Parallel ring with ranked edges: as ring_parallel, but each boundary edge goes to
-// its own lane, and its position in the SimpleCycle iteration order (starting at the
-// first removed vertex's dual[0]) comes from pointer jumping over warp shuffles
-// instead of a walk.  Lane e < E receives edge (*eu -> *ew) at ring position *erank.
-// Returns E, or -1 when the serial replay must decide (the start node is interior,
-// the edges do not form one cycle through it, or more than 32 edges).
-//
-// The boundary test uses S.plm, one 32-bit lane mask per plane (zero between calls):
-// removed triangle `lane` sets its bit on its three planes.  The dual of a convex cell
-// is a triangulated sphere, so an edge {u, w} belongs to exactly two triangles, with
-// opposite orientations; edge u->w of a removed triangle is therefore interior (the
-// other triangle, holding w->u, is removed as well) exactly when another removed
-// triangle holds both u and w.
-template <class T, class SM>
-__device__ __forceinline__ int ring_ranked(SM& S, int lane, int nvf, int nv, int* eu, int* ew,
-                                           int* erank) {
-  using PIdx = typename T::PIdx;
-  const int r = nv - nvf;
-  if (r > 32) return -1;
-  int t0 = 0, t1 = 0, t2 = 0;
-  const unsigned me = 1u << lane;
-  if (lane < r) {
-    const int sl = S.ord[nvf + lane];
-    t0 = S.vd0[sl], t1 = S.vd1[sl], t2 = S.vd2[sl];
-    S.rptr[t0] = (PIdx)T::NONE;
-    S.rptr[t1] = (PIdx)T::NONE;
-    S.rptr[t2] = (PIdx)T::NONE;
-    atomicOr(&S.plm[t0], me);
-    atomicOr(&S.plm[t1], me);
-    atomicOr(&S.plm[t2], me);
-  }
-  const int start = S.vd0[S.ord[nvf]];
-  __syncwarp();
-  bool b01 = false, b12 = false, b20 = false;
-  if (lane < r) {
-    const unsigned m0 = S.plm[t0] & ~me, m1 = S.plm[t1] & ~me, m2 = S.plm[t2] & ~me;
-    b01 = (m0 & m1) == 0u;
-    b12 = (m1 & m2) == 0u;
-    b20 = (m2 & m0) == 0u;
-  }
-  __syncwarp();
-  if (lane < r) S.plm[t0] = 0u, S.plm[t1] = 0u, S.plm[t2] = 0u;
-  const unsigned m01 = __ballot_sync(FULL, b01), m12 = __ballot_sync(FULL, b12),
-                 m20 = __ballot_sync(FULL, b20);
-  const int n01 = __popc(m01), n12 = __popc(m12);
-  const int E = n01 + n12 + __popc(m20);
-  if (E > 32) return -1;
-  // compact the edges: edge index by ballot rank; rptr maps a node to the edge leaving it
-  const unsigned lt = lanemask_lt();
-  const int p01 = __popc(m01 & lt), p12 = n01 + __popc(m12 & lt), p20 = n01 + n12 + __popc(m20 & lt);
-  if (b01) S.ea[p01] = (PIdx)t0, S.eb[p01] = (PIdx)t1, S.rptr[t0] = (PIdx)p01;
-  if (b12) S.ea[p12] = (PIdx)t1, S.eb[p12] = (PIdx)t2, S.rptr[t1] = (PIdx)p12;
-  if (b20) S.ea[p20] = (PIdx)t2, S.eb[p20] = (PIdx)t0, S.rptr[t2] = (PIdx)p20;
-  __syncwarp();
-  int u = 0, w = 0, nx = lane, d = 0;
-  bool broken = false;
-  if (lane < E) {
-    u = S.ea[lane], w = S.eb[lane];
-    nx = S.rptr[w];
-    d = 1;
-    // two boundary edges leave u, or none leaves w
-    broken = S.rptr[u] != (PIdx)lane || nx == (int)T::NONE;
-  }
-  const int se = S.rptr[start];
-  __syncwarp();
-  if (__any_sync(FULL, broken) || se == (int)T::NONE) return -1;
-  // distance from each edge to the start edge along the cycle
-  if (lane == se) nx = lane, d = 0;
-  for (int span = 1; span < E; span <<= 1) {
-    const int dn = __shfl_sync(FULL, d, nx);
-    const int nn = __shfl_sync(FULL, nx, nx);
-    d += dn;
-    nx = nn;
-  }
-  if (__any_sync(FULL, lane < E && nx != se)) return -1;  // not one cycle through the start
-  *eu = u;
-  *ew = w;
-  *erank = d == 0 ? 0 : E - d;
-  return E;
-}
-
 // ------------------------------------------------------------ cell records --
-// A finished cell as the staged integral kernel and the cell export read it, in words:
-// header (np as int32; nv | flags as int32), safety radius, then for the stored planes
-// pl in [pb, np): normals / offsets / generator projections (7 (np - pb) f64); the
-// vertex locations in the reference's order (3 nv f64); the stored planes' right
-// generators (int32); their shift codes and the vertex duals (bytes, the duals as
-// plane indices).
+// A finished cell as the staged integral kernel and the cell export read it, in 8-byte
+// words: header (np as int32; nv | flags as int32), safety radius, then for the stored
+// planes pl in [pb, np) eight words each (normal, offset, the generator's projection, the
+// right generator and shift code as int32), then for the vertices in the reference's order
+// four words each (location, the dual planes as bytes).  Every plane and vertex is read and
+// written as 16-byte pairs (128^3 Poisson cells: the integral kernel 9.9 ms with one array
+// per component, 8.9 ms so).
 //
 // A compact record (the plain builds) leaves out the six boundary planes when no
 // vertex lies on one of them (pb = 6): the integral step reads a plane only through a
@@ -1212,60 +994,50 @@ __device__ __forceinline__ int ring_ranked(SM& S, int lane, int nvf, int nv, int
 constexpr int REC_PB6 = 1 << 16;  // nv word flag: planes start at 6
 
 __host__ __device__ __forceinline__ int64_t rec_words(int np, int nv, int pb = 0) {
-  const int ps = np - pb;
-  return 2 + 7 * (int64_t)ps + 3 * (int64_t)nv + (ps + 1) / 2 + (ps + 3 * nv + 7) / 8;
+  return 2 + 8 * (int64_t)(np - pb) + 4 * (int64_t)nv;
+}
+__device__ __forceinline__ double int_bits(int lo, int hi) { return __hiloint2double(hi, lo); }
+__device__ __forceinline__ void rec_header(double* R, int np, int nv, int pb, double sr) {
+  *reinterpret_cast<double2*>(R) = make_double2(int_bits(np, nv | (pb ? REC_PB6 : 0)), sr);
+}
+// plane k - pb of the record, vertex q of a record with ps planes
+__device__ __forceinline__ void rec_plane(double* R, int k, D3 n, double d, D3 proj, int right, int code) {
+  double2* o = reinterpret_cast<double2*>(R + 2 + 8 * k);
+  o[0] = make_double2(n.x, n.y);
+  o[1] = make_double2(n.z, d);
+  o[2] = make_double2(proj.x, proj.y);
+  o[3] = make_double2(proj.z, int_bits(right, code));
+}
+__device__ __forceinline__ void rec_vertex(double* R, int ps, int q, D3 loc, uint32_t dual) {
+  double2* o = reinterpret_cast<double2*>(R + 2 + 8 * ps + 4 * q);
+  o[0] = make_double2(loc.x, loc.y);
+  o[1] = make_double2(loc.z, int_bits((int)dual, 0));
 }
 
 // Writes the cell held in shared memory (SM layout, see the top of this file, plus
-// bisector_point(J, k, x), the HalfSpace point p of plane k) as a record (full or
-// compact) at words allocated from *counter in rec[0, cap), and its offset to
-// *off_slot.  Returns false when the buffer is full or a plane index does not fit the
-// record's bytes.
+// bisector_point(J, k, x), the HalfSpace point p of plane k) as a full record at words
+// allocated from *counter in rec[0, cap), and its offset to *off_slot.  Returns false
+// when the buffer is full or a plane index does not fit the record's bytes.
 template <class SM>
 __device__ bool write_record(const Job& J, double* rec, int64_t cap, unsigned long long* counter,
-                             int64_t* off_slot, const SM& S, int lane, D3 x, int np, int nv,
-                             double sr, bool full) {
+                             int64_t* off_slot, const SM& S, int lane, D3 x, int np, int nv, double sr) {
   if (np > 255) return false;
-  int pb = 0;
-  if (!full) {
-    bool onb = false;
-    for (int q = lane; q < nv; q += 32) {
-      const int sl = S.ord[q];
-      onb |= S.vd0[sl] < 6 || S.vd1[sl] < 6 || S.vd2[sl] < 6;
-    }
-    pb = __any_sync(FULL, onb) ? 0 : 6;
-  }
-  const int ps = np - pb;
-  const int64_t words = rec_words(np, nv, pb);
+  const int64_t words = rec_words(np, nv);
   unsigned long long off = 0;
   if (lane == 0) off = atomicAdd(counter, (unsigned long long)words);
   off = __shfl_sync(FULL, off, 0);
   if ((int64_t)off + words > cap) return false;
   double* R = rec + off;
-  if (lane == 0) {
-    reinterpret_cast<int32_t*>(R)[0] = np;
-    reinterpret_cast<int32_t*>(R)[1] = nv | (pb ? REC_PB6 : 0);
-    R[1] = sr;
-  }
-  double* nx = R + 2;
-  double *ny = nx + ps, *nz = ny + ps, *dd = nz + ps, *qx = dd + ps, *qy = qx + ps, *qz = qy + ps;
-  double *vxo = qz + ps, *vyo = vxo + nv, *vzo = vyo + nv;
-  int32_t* rt = reinterpret_cast<int32_t*>(vzo + nv);
-  uint8_t* pc = reinterpret_cast<uint8_t*>(vzo + nv + (ps + 1) / 2);
-  uint8_t *d0 = pc + ps, *d1 = d0 + nv, *d2 = d1 + nv;
-  for (int k = lane; k < ps; k += 32) {
-    const int pl = k + pb;
-    const D3 nn = {S.pnx[pl], S.pny[pl], S.pnz[pl]};
-    const D3 pr = plane_project(nn, S.bisector_point(J, pl, x), x);  // Plane::project_onto
-    nx[k] = nn.x, ny[k] = nn.y, nz[k] = nn.z, dd[k] = S.pd[pl];
-    qx[k] = pr.x, qy[k] = pr.y, qz[k] = pr.z;
-    rt[k] = S.pright[pl];
-    pc[k] = S.pcode[pl];
+  if (lane == 0) rec_header(R, np, nv, 0, sr);
+  for (int k = lane; k < np; k += 32) {
+    const D3 nn = {S.pnx[k], S.pny[k], S.pnz[k]};
+    const D3 pr = plane_project(nn, S.bisector_point(J, k, x), x);  // Plane::project_onto
+    rec_plane(R, k, nn, S.pd[k], pr, S.pright[k], S.pcode[k]);
   }
   for (int q = lane; q < nv; q += 32) {
     const int sl = S.ord[q];
-    vxo[q] = S.vx[sl], vyo[q] = S.vy[sl], vzo[q] = S.vz[sl];
-    d0[q] = (uint8_t)S.vd0[sl], d1[q] = (uint8_t)S.vd1[sl], d2[q] = (uint8_t)S.vd2[sl];
+    rec_vertex(R, np, q, {S.vx[sl], S.vy[sl], S.vz[sl]},
+               (uint32_t)S.vd0[sl] | ((uint32_t)S.vd1[sl] << 8) | ((uint32_t)S.vd2[sl] << 16));
   }
   if (lane == 0) *off_slot = (int64_t)off;
   __syncwarp();
@@ -1275,41 +1047,36 @@ __device__ bool write_record(const Job& J, double* rec, int64_t cap, unsigned lo
 // The record at R as the integral step and the cell export read it.  Plane accessors
 // take the plane index pl (>= pb).
 struct RecordView {
-  const double *nx, *ny, *nz, *dd, *qx, *qy, *qz, *vx, *vy, *vz;
-  const int32_t* rt;
-  const uint8_t *pc, *d0, *d1, *d2;
+  const double2 *planes, *verts;  // planes: of plane 0, stored or not
   int np, nv, pb;
   double sr;
   __device__ explicit RecordView(const double* R) {
-    np = __ldg(reinterpret_cast<const int32_t*>(R));
-    const int w = __ldg(reinterpret_cast<const int32_t*>(R) + 1);
+    const double2 h = __ldg(reinterpret_cast<const double2*>(R));
+    const int w = __double2hiint(h.x);
+    np = __double2loint(h.x);
     nv = w & 0xffff;
     pb = (w & REC_PB6) ? 6 : 0;
-    sr = __ldg(R + 1);
-    const int ps = np - pb;
-    // plane arrays indexed by pl - pb
-    nx = R + 2, ny = nx + ps, nz = ny + ps, dd = nz + ps;
-    qx = dd + ps, qy = qx + ps, qz = qy + ps;
-    vx = qz + ps, vy = vx + nv, vz = vy + nv;
-    rt = reinterpret_cast<const int32_t*>(vz + nv);
-    pc = reinterpret_cast<const uint8_t*>(vz + nv + (ps + 1) / 2);
-    d0 = pc + ps, d1 = d0 + nv, d2 = d1 + nv;
+    sr = h.y;
+    planes = reinterpret_cast<const double2*>(R + 2) - 4 * pb;
+    verts = planes + 4 * np;
   }
   __device__ D3 normal(int pl) const {
-    const int k = pl - pb;
-    return {__ldg(nx + k), __ldg(ny + k), __ldg(nz + k)};
+    const double2 a = __ldg(planes + 4 * pl);
+    return {a.x, a.y, __ldg(&planes[4 * pl + 1].x)};
   }
-  __device__ double d(int pl) const { return __ldg(dd + pl - pb); }
+  __device__ double d(int pl) const { return __ldg(&planes[4 * pl + 1].y); }
   __device__ D3 proj(int pl) const {
-    const int k = pl - pb;
-    return {__ldg(qx + k), __ldg(qy + k), __ldg(qz + k)};
+    const double2 a = __ldg(planes + 4 * pl + 2);
+    return {a.x, a.y, __ldg(&planes[4 * pl + 3].x)};
   }
-  __device__ int right(int pl) const { return __ldg(rt + pl - pb); }
-  __device__ int code(int pl) const { return __ldg(pc + pl - pb); }
-  __device__ int dual(int q, int i) const {
-    return i == 0 ? __ldg(d0 + q) : (i == 1 ? __ldg(d1 + q) : __ldg(d2 + q));
+  __device__ int right(int pl) const { return __ldg(reinterpret_cast<const int*>(&planes[4 * pl + 3].y)); }
+  __device__ int code(int pl) const { return __ldg(reinterpret_cast<const int*>(&planes[4 * pl + 3].y) + 1); }
+  __device__ uint32_t duals(int q) const { return (uint32_t)__ldg(reinterpret_cast<const int*>(&verts[2 * q + 1].y)); }
+  __device__ int dual(int q, int i) const { return (int)((duals(q) >> (8 * i)) & 0xffu); }
+  __device__ D3 loc(int q) const {
+    const double2 a = __ldg(verts + 2 * q);
+    return {a.x, a.y, __ldg(&verts[2 * q + 1].x)};
   }
-  __device__ D3 loc(int q) const { return {__ldg(vx + q), __ldg(vy + q), __ldg(vz + q)}; }
 };
 
 // Projection of x on the line of planes dual[i] & dual[i+1] of vertex q:

@@ -68,6 +68,43 @@ __host__ __device__ __forceinline__ double signed_area_tri(D3 v0, D3 v1, D3 v2, 
   return sqrt(dot(n, n)) * sign;
 }
 
+#ifdef __CUDACC__
+// Several correctly rounded quotients by one divisor, from its correctly rounded
+// reciprocal y = RN(1 / b): with q a faithful rounding of a / b and the residual
+// r = a - b q exact (one FMA), RN(q + r y) is RN(a / b) (P. Markstein, Computation of
+// elementary functions on the IBM RISC System/6000 processor, IBM J. Res. Dev. 34, 1990;
+// Muller et al., Handbook of Floating-Point Arithmetic, division by Newton iterations).
+// RN(a y) is within two ulps, the first correction makes it faithful and the second
+// correct.  The theorem needs exponents away from under- and overflow: operands outside
+// 2^-400 .. 2^400 (zeros among them) take the division itself.
+__device__ __forceinline__ bool mid_range(double v) {
+  return ((unsigned)(__double2hiint(v) & 0x7fffffff) - ((1023u - 400u) << 20)) < (800u << 20);
+}
+// a / b per component when b and the components are mid-range; false (and nothing
+// written) otherwise.
+__device__ __forceinline__ bool quotients(D3 a, double b, D3* out) {
+  if (!(mid_range(b) && mid_range(a.x) && mid_range(a.y) && mid_range(a.z))) return false;
+  const double y = __drcp_rn(b);
+  double qx = a.x * y, qy = a.y * y, qz = a.z * y;
+#pragma unroll
+  for (int i = 0; i < 2; i++) {
+    qx = __fma_rn(__fma_rn(-b, qx, a.x), y, qx);
+    qy = __fma_rn(__fma_rn(-b, qy, a.y), y, qy);
+    qz = __fma_rn(__fma_rn(-b, qz, a.z), y, qz);
+  }
+  *out = {qx, qy, qz};
+  return true;
+}
+// The numerator vector and determinant of intersect3.
+__device__ __forceinline__ D3 intersect3_parts(D3 n0, double d0, D3 n1, double d1, D3 n2, double d2, double* det) {
+  *det = det_cols(n0, n1, n2);
+  const D3 a = scale(d0, cross(n1, n2));
+  const D3 b = scale(d1, cross(n2, n0));
+  const D3 c = scale(d2, cross(n0, n1));
+  return add(add(a, b), c);
+}
+#endif
+
 // Dimensionality::vector_is_valid (voronoi.rs:42-49)
 __host__ __device__ __forceinline__ bool vector_is_valid(int dim, D3 v) {
   if (dim == 1) return v.y == 0.0 && v.z == 0.0;

@@ -156,6 +156,7 @@ struct StageJob {
   unsigned long long* rec_counter;
   int32_t full_records;       // 1: full records (export builds), 0: compact (write_record)
   int32_t box;                // 1: the clip kernel decides box-corner band tests itself
+  int32_t per_warp;           // clip kernel: cells that a warp builds at a time
   unsigned int* work;         // [3] work counters of the shell, clip and integral kernels
   int32_t* retry_list;        // positions the next round (wide round, fused kernel) takes
   unsigned int* retry_count;
