@@ -19,7 +19,7 @@
 // instruction fetch: the loop's code has to stay within the 32 KB first-level instruction
 // cache, so what is rarely needed is kept out of line and loops are not unrolled.
 // 128^3 Poisson cells: with one warp per cell (28 warps per SM, 15.2 k warp-instructions
-// per cell) 34.1 ms, in this form (7 k) 21.6 ms; replacing a warp's finished cells one by
+// per cell) 34.1 ms, in this form (6.9 k) 20.3 ms; replacing a warp's finished cells one by
 // one instead of all four together (fuller warps, but the once-per-cell code runs four
 // times as often) 36 ms.
 #include <algorithm>
@@ -92,9 +92,15 @@ struct GroupPlanes {
   __device__ __forceinline__ D3 normal(int k) const { return {pxy[k].x, pxy[k].y, pzd[k].x}; }
   __device__ __forceinline__ double d(int k) const { return pzd[k].y; }
   // intersect_planes (geometry.rs:68-76) of the dual planes, out of the hot loop's code
-  __device__ __noinline__ bool intersect(uint32_t dual, D3* loc) const {
+  struct Meet {
+    D3 loc;
+    bool ok;
+  };
+  __device__ __noinline__ Meet intersect(uint32_t dual) const {
     const int i = dual & 0xff, j = (dual >> 8) & 0xff, k = (dual >> 16) & 0xff;
-    return intersect3(normal(i), d(i), normal(j), d(j), normal(k), d(k), loc);
+    Meet m = {{0.0, 0.0, 0.0}, false};
+    m.ok = intersect3(normal(i), d(i), normal(j), d(j), normal(k), d(k), &m.loc);
+    return m;
   }
   __device__ __noinline__ D3 intersect_loc(uint32_t dual) const {
     D3 l = {0.0, 0.0, 0.0};
@@ -106,7 +112,10 @@ struct GroupPlanes {
     const int i = dual & 0xff, j = (dual >> 8) & 0xff, k = (dual >> 16) & 0xff;
     double det;
     const D3 s = intersect3_parts(normal(i), d(i), normal(j), d(j), normal(k), d(k), &det);
-    return quotients(s, det, loc) || intersect(dual, loc);
+    if (quotients(s, det, loc)) return true;
+    const Meet m = intersect(dual);
+    *loc = m.loc;
+    return m.ok;
   }
 };
 
@@ -226,21 +235,19 @@ __device__ __noinline__ double exact_radius(const SM& S, int gl, int nv, float m
   return 2.0 * sqrt(group_max<G>(m));
 }
 
-// Candidate k of a group (`near`) that is not certainly within the safety radius, with
-// the f32 distance d32 (rounded up), or the list's end: the cell's result when this ends
-// it, -1 when the candidate is to be clipped.  su_hi bounds the safety radius; the f64
-// value is computed where that leaves it open.  Called by the whole warp.
+// Candidate k of a group (`near`) whose f32 distance leaves open whether it is within the
+// safety radius, or the list's end: the cell's result when this ends it, -1 when the
+// candidate is to be clipped.  su_hi bounds the safety radius.  Called by the whole warp.
 template <int G, class SM>
 __device__ __noinline__ int at_radius(const Job& J, const StageJob& SJ, const SM& S, const uint32_t* list, int gl,
-                                      int item, int info, bool near, int k, int nv, float d32, float su_hi, float m2,
+                                      int item, int info, bool near, int k, int nv, float su_hi, float m2,
                                       D3 x, int dim) {
   const int ncand = info & 0x3fffffff;
   const bool exhausted = (info >> 30) & 1;
   const double rad = near && k == ncand ? SJ.rad[item] : 0.0;
   int got = -1;
-  if (near && (k == ncand ? exhausted || (double)su_hi < rad * (1.0 - 1e-6) : d32 > su_hi && d32 < INFINITY)) {
-    // certainly beyond it (convex_cell.rs:343-345), or the whole stream was consumed
-    got = CELL_DONE;
+  if (near && k == ncand && (exhausted || (double)su_hi < rad * (1.0 - 1e-6))) {
+    got = CELL_DONE;  // the whole stream was consumed, or the list reaches beyond the radius
     near = false;
   }
   if (__any_sync(FULL, near)) {
@@ -366,11 +373,11 @@ __device__ __noinline__ void swap_remove_any(SM& S, int gl, int r, int rmax, int
 }
 
 // The vertices (chunks `open` of this lane) that the filter left open against candidate k,
-// whose half-space is plane np: returns the chunks of those removed, bit 31 set when one
-// needs the multi-limb predicate.
+// whose half-space is plane np: returns the chunks of those removed (bits 0-15), the number
+// of box-corner tests (from bit 16), and bit 31 when one needs the multi-limb predicate.
 template <class T, int PREC, bool BOX, class SM>
 __device__ __noinline__ unsigned undecided(const Job& J, const SM& S, const uint32_t* list, int gl, int np,
-                                           int k, unsigned open, D3 x, unsigned* n_ex) {
+                                           int k, unsigned open, D3 x) {
   const D3 n = S.normal(np);
   const double d = S.d(np);
   const D3 g = cand_loc(J, __ldg(list + k));
@@ -388,7 +395,7 @@ __device__ __noinline__ unsigned undecided(const Job& J, const SM& S, const uint
     if (band) {
       if constexpr (BOX) {
         if (!group_box_zero(J, S, list, S.dual(q), x, g)) out |= 1u << 31;
-        *n_ex += 1u;
+        out += 1u << 16;
       } else {
         out |= 1u << 31;
       }
@@ -401,11 +408,9 @@ __device__ __noinline__ unsigned undecided(const Job& J, const SM& S, const uint
 // node is interior: the reference joins the triangles one by one, each time the first (in
 // an order that its swaps change) that extends the cycle, and moves the start to the node
 // before it in the triangle that closes its fan.  Triangle gl: nodes du, M and N as in the
-// clip kernel (N zero in groups that do not take part); r triangles.  Called by the whole
-// warp.  The cycle holds the reversed edge a of a waiting triangle when N_a meets the
+// clip kernel (N zero in groups that do not take part).  Called by the whole warp.  The cycle holds the reversed edge a of a waiting triangle when N_a meets the
 // joined lanes A, and its node a when M_a does.
-__device__ __noinline__ void ring_start(uint32_t du, uint32_t M, uint32_t N, int gl, int gbase, int r, int* start_io) {
-  int start = *start_io;
+__device__ __noinline__ int ring_start(uint32_t du, uint32_t M, uint32_t N, int gl, int gbase, int start) {
   uint32_t A = 0x010101u;  // in all three bytes
   int at = gl;             // the lane of the triangle at position gl
   if (gl == 0) N = 0u;     // the first triangle is the cycle
@@ -435,16 +440,16 @@ __device__ __noinline__ void ring_start(uint32_t du, uint32_t M, uint32_t N, int
       if ((w >> 24) != 0u && start == (int)((w >> 8) & 0xff)) start = w & 0xff;
     }
   }
-  if (r > 0) *start_io = start;
+  return start;
 }
 
 // The ring of a group (`on`) that removes more vertices, or gets more edges, than it has
 // lanes: compute_boundary + SimpleCycle through shared memory (S.ring: successors; S.rd:
 // the removed triangles, which the ring's nodes replace in cycle order).  Called by the
-// whole warp.  Returns false when a triangle cannot be joined.
+// whole warp.  Returns the number of edges, bit 16 set when the ring's start moved; 0 when
+// a triangle cannot be joined.
 template <class T, class SM>
-__device__ __noinline__ bool ring_wide(SM& S, int gl, int gbase, bool on, int r, int* start_out, int* E_out,
-                                       bool* moved_out) {
+__device__ __noinline__ unsigned ring_wide(SM& S, int gl, int gbase, bool on, int r) {
   constexpr int G = T::G;
   constexpr unsigned GM = G == 32 ? FULL : ((1u << G) - 1u);
   uint8_t* const rptr = reinterpret_cast<uint8_t*>(S.ring);
@@ -506,10 +511,9 @@ __device__ __noinline__ bool ring_wide(SM& S, int gl, int gbase, bool on, int r,
     __syncwarp(GM << gbase);
 #pragma unroll 1
     for (int i = gl; i < (T::PMAX + 4) / 4; i += G) S.ring[i] = ~0u;
-    *start_out = start, *E_out = E, *moved_out = moved;
   }
   __syncwarp();
-  return ok;
+  return ok ? (unsigned)E | (moved ? 1u << 16 : 0u) : 0u;
 }
 
 // Writes the finished cells (`on`) of a warp's groups as records (see rec_words), their
@@ -726,9 +730,13 @@ __global__ void __launch_bounds__(32 * T::WARPS, T::MINB)
             cc = S.wc[k & (WIN - 1)], cd = S.wc[(k + 1) & (WIN - 1)];
           }
           // the list's end, a degenerate distance, or not certainly within the safety radius
-          const bool near = search && !(cc.y < su_lo);
+          bool near = search && !(cc.y < su_lo);
+          if (near && cc.y > su_hi && cc.y < INFINITY) {  // certainly beyond it (convex_cell.rs:343-345)
+            res = CELL_DONE;
+            near = search = act = false;
+          }
           if (__any_sync(FULL, near)) {
-            const int got = at_radius<G>(J, SJ, S, list, gl, item, info, near, k, nv, cc.y, su_hi, m2, x, dim);
+            const int got = at_radius<G>(J, SJ, S, list, gl, item, info, near, k, nv, su_hi, m2, x, dim);
             if (near && got >= 0) {
               res = got;
               if (got == CELL_ERROR) err = MV_ERR_DEGENERATE;  // convex_cell.rs:342
@@ -828,9 +836,10 @@ __global__ void __launch_bounds__(32 * T::WARPS, T::MINB)
         bool hard = false;
         if (open) {
           if constexpr (FILT) n_und += __popc(open);
-          const unsigned got = undecided<T, PREC, BOX>(J, S, list, gl, np, k, open, x, &n_ex);
+          const unsigned got = undecided<T, PREC, BOX>(J, S, list, gl, np, k, open, x);
           hard = got >> 31;
-          rl |= got & 0x7fffffffu;
+          n_ex += (got >> 16) & 0x7fffu;
+          rl |= got & 0xffffu;
         }
         if ((__ballot_sync(FULL, hard) & gmask) != 0u && hit) {
           res = CELL_EXACT;
@@ -909,7 +918,7 @@ __global__ void __launch_bounds__(32 * T::WARPS, T::MINB)
         moved = hit && !wide && next[start] == RING_NONE;
         if (__any_sync(FULL, moved)) {
           if (!moved) N = 0u;
-          ring_start(du, M, N, gl, gbase, moved ? r : 0, &start);
+          start = ring_start(du, M, N, gl, gbase, start);
         }
       }
       int u, w;
@@ -935,8 +944,9 @@ __global__ void __launch_bounds__(32 * T::WARPS, T::MINB)
       if (__any_sync(FULL, wide)) {
         // more removed vertices or ring edges than lanes (or an order that only the reference's
         // own loop decides): the ring through shared memory
-        const bool ok = ring_wide<T>(S, gl, gbase, wide && hit, r, &start, &E, &moved);
-        if (wide && hit && !ok) {
+        const unsigned got = ring_wide<T>(S, gl, gbase, wide && hit, r);
+        if (wide) E = got & 0xffff, moved = got >> 16;
+        if (wide && hit && got == 0u) {
           res = CELL_ERROR, err = MV_ERR_RING;
           hit = act = false;
         }
