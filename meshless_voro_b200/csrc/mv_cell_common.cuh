@@ -439,8 +439,11 @@ __device__ __noinline__ int gather_shell_impl(const Job& J, ShellBuf<CMAX>& B, i
     int G = J.G[i];
     bool wrap = J.periodic && i < J.dim;
     int umin = wrap ? -G : 0, umax = wrap ? 2 * G - 1 : G - 1;
-    double fl = floor((xa[i] - R - J.ga[i]) * J.ginv[i]) - 1.0;
-    double fh = floor((xa[i] + R - J.ga[i]) * J.ginv[i]) + 1.0;
+    // the cells that hold [x - R, x + R], widened against the rounding of the cell index as
+    // the cell boxes are (by no more: a first shell then has at most 32 rows of cells, one
+    // per lane, where a spare cell on each side gave it two passes of rows)
+    double fl = floor((xa[i] - R - J.geps[i] - J.ga[i]) * J.ginv[i]);
+    double fh = floor((xa[i] + R + J.geps[i] - J.ga[i]) * J.ginv[i]);
     lo[i] = fl < (double)umin ? umin : (int)fl;
     hi[i] = fh > (double)umax ? umax : (int)fh;
     if (lo[i] > umin || hi[i] < umax) all = false;

@@ -42,10 +42,10 @@ __device__ __forceinline__ int stage_pos(const StageJob& SJ, int item) {
 }
 
 // ------------------------------------------------------------------- shell --
-// Bitonic sort of 32 * EPL entries in registers (element i = lane + 32 e in slot e of
-// every lane) by a 32-bit key alone, carrying the list word; as sort_regs.
+// Bitonic sort of 32 * EPL distinct 32-bit keys in registers (element i = lane + 32 e in
+// slot e of every lane): one shuffle and one minimum or maximum per exchange.
 template <int EPL>
-__device__ __forceinline__ void sort_regs_key(uint32_t (&key)[EPL], uint32_t (&val)[EPL], int lane) {
+__device__ __forceinline__ void sort_regs_key(uint32_t (&key)[EPL], int lane) {
 #pragma unroll
   for (int k = 2; k <= 32 * EPL; k <<= 1) {
 #pragma unroll
@@ -56,50 +56,51 @@ __device__ __forceinline__ void sort_regs_key(uint32_t (&key)[EPL], uint32_t (&v
           const int pe = e ^ (j >> 5);
           if (pe > e) {
             const bool asc = ((32 * e) & k) == 0;
-            if ((key[e] > key[pe]) == asc) {
-              const uint32_t tk = key[e];
-              const uint32_t tv = val[e];
-              key[e] = key[pe], val[e] = val[pe];
-              key[pe] = tk, val[pe] = tv;
-            }
+            const uint32_t a = key[e], b = key[pe];
+            key[e] = asc ? min(a, b) : max(a, b);
+            key[pe] = asc ? max(a, b) : min(a, b);
           }
         }
       } else {
 #pragma unroll
         for (int e = 0; e < EPL; e++) {
-          const uint32_t ok = __shfl_xor_sync(FULL, key[e], j);
-          const uint32_t ov = __shfl_xor_sync(FULL, val[e], j);
-          const bool asc = (((lane + 32 * e) & k) == 0);
-          const bool lower = (lane & j) == 0;
-          if ((key[e] > ok) == (lower == asc)) key[e] = ok, val[e] = ov;
+          const uint32_t o = __shfl_xor_sync(FULL, key[e], j);
+          const bool low = ((((lane + 32 * e) & k) == 0) == ((lane & j) == 0));
+          key[e] = low ? min(key[e], o) : max(key[e], o);
         }
       }
     }
   }
 }
 
-// Sorts the gathered shell (cnt <= 32 EPL entries; B.tie holds the shift codes) in
-// registers and writes it as sorted position * 27 + shift code; returns whether the
-// nearest entry is the generator itself (sorted position spos, no shift).  The entries are sorted by their
-// squared distance rounded down to f32 (a monotone map, so distinct keys order the
-// entries as their squared distances do); only when two keys are equal (distances
-// within an f32 ulp, or equal as in lattice-like inputs) is the shell sorted again by
-// (squared distance, original index, shift code), the stream's full order.
+// Sorts the gathered shell (cnt <= 32 EPL entries with squared distances below R2; B.tie
+// holds the shift codes) in registers and writes it as sorted position * 27 + shift code;
+// returns whether the nearest entry is the generator itself (sorted position spos, no
+// shift).  An entry's key is its squared distance as a 25-bit fraction of R2 above its
+// index in the shell: one word to compare and move per entry (a distance word and a list
+// word before; with one row pass per query, see gather_shell: 128^3 Poisson cells 10.8 ->
+// 7.6 ms), which orders the entries as
+// their squared distances do (the fraction is a monotone function of them) unless two
+// fractions are equal (distances within 2^-25 R2, or equal as in lattice-like inputs; one
+// uniform cell in some thousands); the shell is then sorted again by (squared distance,
+// original index, shift code), the stream's full order.
 template <int EPL>
 __device__ __forceinline__ bool sort_and_write(const Job& J, const ShellBuf<SHELL_CMAX>& B, int lane,
-                                               int cnt, int self, int spos, uint32_t* out) {
+                                               int cnt, double R2, int self, int spos, uint32_t* out) {
   uint32_t key[EPL];
-  uint32_t val[EPL];
+  const double scale = (double)(1 << 25) / R2;
 #pragma unroll
   for (int e = 0; e < EPL; e++) {
     const int i = lane + 32 * e;
-    // d2 >= 0 is finite: its f32 bit pattern orders as the value, below the padding
-    key[e] = i < cnt ? __float_as_uint(__double2float_rd(__longlong_as_double((long long)B.key[i])))
-                     : ~0u;
-    val[e] = i < cnt ? (uint32_t)B.cpos[i] * 27u + B.tie[i] : 0u;
+    // 0 <= d2 < R2; the rounded product may reach 2^25
+    const uint32_t f =
+        i < cnt ? min(__double2uint_rz(__longlong_as_double((long long)B.key[i]) * scale), (1u << 25) - 1u)
+                : (1u << 25) - 1u;
+    key[e] = (f << 7) | (uint32_t)i;
   }
-  sort_regs_key<EPL>(key, val, lane);
-  // equal keys end next to each other: element i against i + 1
+  sort_regs_key<EPL>(key, lane);
+  // equal fractions end next to each other: element i against i + 1 (padding, with the
+  // largest fraction and indices from cnt on, sorts behind every entry)
   bool dup = false;
 #pragma unroll
   for (int e = 0; e < EPL; e++) {
@@ -107,7 +108,7 @@ __device__ __forceinline__ bool sort_and_write(const Job& J, const ShellBuf<SHEL
     const uint32_t wrap = __shfl_sync(FULL, key[e + 1 < EPL ? e + 1 : e], 0);
     const uint32_t next = lane < 31 ? nx : wrap;
     const int i = lane + 32 * e;
-    dup |= (i + 1 < cnt) && (lane < 31 || e + 1 < EPL) && key[e] == next;
+    dup |= (i + 1 < cnt) && (key[e] >> 7) == (next >> 7);
   }
   if (__any_sync(FULL, dup)) {
     unsigned long long dkey[EPL];
@@ -128,12 +129,15 @@ __device__ __forceinline__ bool sort_and_write(const Job& J, const ShellBuf<SHEL
     }
     return (int)(__shfl_sync(FULL, tie[0], 0) / 27u) == self;
   }
+  uint32_t first = 0u;
 #pragma unroll
   for (int e = 0; e < EPL; e++) {
-    const int i = lane + 32 * e;
-    if (i < cnt) out[i] = val[e];
+    const int i = lane + 32 * e, at = (int)(key[e] & 127u);
+    const uint32_t v = (uint32_t)B.cpos[at] * 27u + B.tie[at];
+    if (i < cnt) out[i] = v;
+    if (e == 0) first = v;
   }
-  return __shfl_sync(FULL, val[0], 0) == (uint32_t)spos * 27u + 13u;
+  return __shfl_sync(FULL, first, 0) == (uint32_t)spos * 27u + 13u;
 }
 
 template <int WARPS, bool MULTI>
@@ -187,11 +191,11 @@ __global__ void __launch_bounds__(32 * WARPS, MV_SHELL_MINB)
     uint32_t* out = SJ.cand + (int64_t)item * SJ.cstride;
     bool self_first;
     if (cnt <= 32)
-      self_first = sort_and_write<1>(J, B, lane, cnt, self, spos, out);
+      self_first = sort_and_write<1>(J, B, lane, cnt, R * R, self, spos, out);
     else if (cnt <= 64)
-      self_first = sort_and_write<2>(J, B, lane, cnt, self, spos, out);
+      self_first = sort_and_write<2>(J, B, lane, cnt, R * R, self, spos, out);
     else
-      self_first = sort_and_write<4>(J, B, lane, cnt, self, spos, out);
+      self_first = sort_and_write<4>(J, B, lane, cnt, R * R, self, spos, out);
     // the first neighbour must be the generator itself (convex_cell.rs:325-329); the
     // fused kernel reports the error otherwise
     if (lane == 0) {
