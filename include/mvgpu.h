@@ -372,6 +372,27 @@ int mv_voronoi_build_noalloc(const double* d_generators, const uint8_t* d_mask, 
                              int periodic, const mv_options* opts, mv_device_voronoi* out,
                              int64_t face_capacity, int64_t connection_capacity);
 
+/* ---- copies of results (no counterpart in the reference crate) ----
+ *
+ * Copies arrays of a host result out of the context's arena into the caller's own memory,
+ * widening indices on the way, on several threads.  The copies must not overlap.  Callable
+ * from any thread; touches neither the GPU nor a context. */
+enum {
+  MV_COPY_1 = 1,           /* elements of 1, 4 and 8 bytes as they are                */
+  MV_COPY_4 = 2,
+  MV_COPY_8 = 3,
+  MV_COPY_I32_TO_I64 = 4,
+  MV_COPY_U8_TO_I32 = 5
+};
+typedef struct mv_copy {
+  const void* src;
+  void* dst;
+  int64_t count;           /* elements                                                */
+  int32_t kind;            /* MV_COPY_*                                               */
+  int32_t reserved;
+} mv_copy;
+int mv_copy_arrays(const mv_copy* copies, int count);
+
 /* The reference's shift vector for a face shift code (rtree_nn.rs:27-33): component i
  * is m_i * width_i for m_i != 0 and -0.0 for m_i == 0, with (m_x, m_y, m_z) decoded
  * from code = (m_x+1) + 3(m_y+1) + 9(m_z+1).  Code 13 (no shift) gives all -0.0. */

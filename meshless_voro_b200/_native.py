@@ -8,6 +8,8 @@ from __future__ import annotations
 import ctypes as C
 import os
 
+import numpy as np
+
 _HERE = os.path.dirname(os.path.abspath(__file__))
 # MVGPU_LIBRARY selects another build of the library (e.g. a tuning variant)
 LIB_PATH = os.environ.get("MVGPU_LIBRARY") or os.path.join(_HERE, "_lib", "libmvgpu.so")
@@ -43,7 +45,7 @@ EXPORTED = (
     "mv_context_build", "mv_voronoi_build", "mv_voronoi_build_partial", "mv_voronoi_free",
     "mv_shift_from_code", "mv_voronoi_build_noalloc", "mv_context_build_cells_device",
     "mv_context_build_cells", "mv_context_build_batch_device", "mv_context_build_batch",
-    "mv_tuning_set", "mv_tuning_lookup", "mv_tuning_count",
+    "mv_tuning_set", "mv_tuning_lookup", "mv_tuning_count", "mv_copy_arrays",
 )
 
 
@@ -113,6 +115,12 @@ class Job(C.Structure):
     _fields_ = [("n", C.c_int64), ("anchor", C.c_double * 3), ("width", C.c_double * 3),
                 ("dimensionality", C.c_int32), ("periodic", C.c_int32), ("has_mask", C.c_int32),
                 ("reserved", C.c_int32)]
+
+
+class Copy(C.Structure):
+    """mv_copy: one array of mv_copy_arrays."""
+    _fields_ = [("src", C.c_void_p), ("dst", C.c_void_p), ("count", C.c_int64),
+                ("kind", C.c_int32), ("reserved", C.c_int32)]
 
 
 class TuningEntry(C.Structure):
@@ -205,6 +213,8 @@ def lib():
         L.mv_tuning_lookup.restype = C.c_int
         L.mv_tuning_count.argtypes = []
         L.mv_tuning_count.restype = C.c_int
+        L.mv_copy_arrays.argtypes = [C.POINTER(Copy), C.c_int]
+        L.mv_copy_arrays.restype = C.c_int
         _lib = L
     return _lib
 
@@ -219,6 +229,28 @@ class MvError(RuntimeError):
         if error_cell >= 0:
             msg += f" (cell {error_cell})"
         super().__init__(msg)
+
+
+# (element size in the library's array, numpy type of the copy) -> mv_copy kind
+_COPY_KINDS = {(8, 8): 3, (4, 4): 2, (1, 1): 1, (4, 8): 4, (1, 4): 5}
+
+
+class ArrayCopies:
+    """Copies of library arrays into new numpy arrays, gathered and then made together
+    (mv_copy_arrays).  Integers may widen: int32 to int64, uint8 to int32."""
+
+    def __init__(self):
+        self._items = []
+
+    def take(self, ptr, count: int, itemsize: int, dtype, shape=None) -> np.ndarray:
+        """A new array that run() fills with `count` elements of `itemsize` bytes at ptr."""
+        out = np.empty(count, dtype=dtype)
+        address = C.cast(ptr, C.c_void_p).value
+        self._items.append((address, out.ctypes.data, count, _COPY_KINDS[itemsize, out.itemsize], 0))
+        return out.reshape(shape) if shape else out
+
+    def run(self):
+        check(lib().mv_copy_arrays((Copy * len(self._items))(*self._items), len(self._items)))
 
 
 def check(status: int, error_cell: int = -1):

@@ -21,7 +21,7 @@ OBJ_DIR = os.path.join(LIB_DIR, "obj")
 LIB = os.path.join(LIB_DIR, "libmvgpu.so")
 
 SOURCES = ["mv_api.cu", "mv_cells.cu", "mv_grid.cu", "mv_noalloc.cu", "mv_staged.cu", "mv_clip.cu", "mv_export.cu",
-           "mv_tuning.cu"]
+           "mv_tuning.cu", "mv_host.cu"]
 HEADERS = ["mv_geom.cuh", "mv_exact.cuh", "mv_internal.h", "mv_cell_common.cuh", "mv_tuning_table.h"]
 
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")

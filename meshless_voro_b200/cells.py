@@ -55,9 +55,9 @@ class CellsArrays:
                 return None
             if count == 0:
                 return np.zeros(shape, dtype=ctype)
-            p = C.cast(ptr, C.POINTER(np.ctypeslib.as_ctypes_type(ctype)))
-            return np.ctypeslib.as_array(p, shape=(count,)).copy().reshape(shape)
+            return copies.take(ptr, count, np.dtype(ctype).itemsize, ctype, shape)
 
+        copies = N.ArrayCopies()
         out = CellsArrays(
             n_cells=n,
             plane_offset=arr(h.cell_plane_offset, n + 1, np.int64, (n + 1,)),
@@ -77,6 +77,7 @@ class CellsArrays:
             out.face_plane = arr(h.face_plane, Fc, np.int32, (Fc,))
             out.face_vertex_offset = arr(h.face_vertex_offset, Fc + 1, np.int64, (Fc + 1,))
             out.face_vertices = arr(h.face_vertices, FV, np.int32, (FV,))
+        copies.run()
         return out
 
 

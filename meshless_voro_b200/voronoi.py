@@ -349,10 +349,12 @@ class VoronoiArrays:
             if count == 0 or not ptr:
                 a = np.zeros(0 if shape is None else (0,) + shape[1:], dtype=dtype)
                 return a
+            if copy:
+                return copies.take(ptr, count, C.sizeof(ptr._type_), dtype, shape)
             a = np.ctypeslib.as_array(ptr, shape=(count,))
-            a = a.astype(dtype, copy=True) if copy else a
             return a.reshape(shape) if shape else a
 
+        copies = N.ArrayCopies()
         dim = int(hv.dimensionality)
         loc = generators.copy()
         if dim == 1:
@@ -362,7 +364,7 @@ class VoronoiArrays:
         if mask_u8 is not None:
             loc[mask_u8 == 0] = 0.0
         has_csr = bool(hv.cell_face_offset)
-        return VoronoiArrays(
+        out = VoronoiArrays(
             n_cells=n, anchor=np.array(hv.anchor[:]), width=np.array(hv.width[:]),
             dimensionality=dim, periodic=bool(hv.periodic),
             cell_volume=arr(hv.cell_volume, n, np.float64),
@@ -379,6 +381,8 @@ class VoronoiArrays:
             face_shift_code=arr(hv.face_shift_code, F, np.int32),
             cell_face_connections=arr(hv.cell_face_connections, Cn, np.int64) if has_csr else None,
         )
+        copies.run()
+        return out
 
 
 class VoronoiCell:
