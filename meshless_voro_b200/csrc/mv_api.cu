@@ -56,11 +56,11 @@ int64_t stage_record_words(int np, int nv);
 // mv_grid.cu
 void launch_prep(const double* xyz, int n, int dim, double* gen, unsigned long long* ext_keys,
                  double* ext, int* bad, cudaStream_t st);
-void launch_grid_coarse(const double* gen, int n, const int G[3], const double a[3],
+int launch_grid_coarse(const double* gen, int n, const int G[3], const double a[3],
                         const double inv[3], int32_t* cid, int32_t* count, int32_t* start,
                         int32_t* dflag, int32_t* dprefix, int dim, long long* scan_tmp, cudaStream_t st);
 size_t grid_dense_sort_bytes(int n, int64_t ncell);
-void launch_batch_grid(const double* xyz, int n, const int32_t* pos, const int32_t* cbase, int nj,
+int launch_batch_grid(const double* xyz, int n, const int32_t* pos, const int32_t* cbase, int nj,
                        const BatchGrid* bg, int64_t ncell, double* gen, unsigned long long* ext_keys,
                        double* ext, int* bad, int32_t* cid, int32_t* count, int32_t* start,
                        int32_t* dflag, int32_t* dprefix, long long* scan_tmp, cudaStream_t st);
@@ -69,12 +69,6 @@ cudaError_t launch_batch_sort(const double* gen, int n, const int32_t* pos, cons
                               unsigned long long* key_a, unsigned long long* key_b, int32_t* val_a,
                               int32_t* val_b, void* sort_tmp, size_t sort_bytes, double* sx, double* sy,
                               double* sz, int32_t* sid, uint32_t* fkey, int32_t* start, cudaStream_t st);
-void launch_batch_csr(const FaceArrays& f, int64_t F, const int64_t* face_off, const int32_t* face_count,
-                      int n, const int32_t* pos, int nj, int32_t* in_count, int32_t* conn_count,
-                      cudaStream_t st);
-void launch_batch_csr_fill(const FaceArrays& f, int64_t F, const int64_t* face_off, const int64_t* conn_off,
-                           const int32_t* in_count, int32_t* cursor, int n, const int32_t* pos, int nj,
-                           int32_t* conn, cudaStream_t st);
 void launch_batch_localize(FaceArrays& f, int64_t F, const int64_t* face_off, int64_t* conn_off,
                            const int32_t* conn_count, int32_t* conn, int n, const int32_t* pos, int nj,
                            int64_t* fbase, int64_t* cbase_conn, cudaStream_t st);
@@ -86,13 +80,16 @@ cudaError_t launch_grid_dense(const double* gen, int n, const int G[3], const do
 void launch_scatter(const double* gen, int n, const int32_t* cid, const int32_t* start,
                     int32_t* fill, double* sx, double* sy, double* sz, int32_t* sid, cudaStream_t st);
 size_t scan_tmp_elems(int64_t n);
-void scan_i32_to_i64(const int32_t* in, int64_t n, int64_t* out, long long* tmp, cudaStream_t st);
-void launch_reorder(const FaceArrays& stage, int64_t F, const int64_t* stage_off,
-                    const int64_t* face_off, const FaceArrays& out, cudaStream_t st);
-void launch_csr_counts(const FaceArrays& f, int64_t F, const int32_t* face_count, int n,
-                       int32_t* in_count, int32_t* conn_count, cudaStream_t st);
-void launch_csr_fill(const FaceArrays& f, int64_t F, const int64_t* face_off, const int64_t* conn_off,
-                     const int32_t* in_count, int32_t* cursor, int n, int32_t* conn, cudaStream_t st);
+int scan_i32_to_i64(const int32_t* in, int64_t n, int64_t* out, long long* tmp, cudaStream_t st);
+int scan_rows_i32_to_i64(const int32_t* in, int64_t n, int rows, int64_t stride, int64_t* out, long long* tmp,
+                         cudaStream_t st);
+void launch_reorder(const FaceArrays& stage, int n, const int64_t* stage_off, const int64_t* face_off,
+                    const FaceArrays& out, int32_t* in_count, const int32_t* pos, int nj, cudaStream_t st);
+int launch_csr_offsets(const int32_t* face_count, const int32_t* in_count, int64_t n, int32_t* conn_count,
+                       int64_t* conn_off, long long* scan_tmp, cudaStream_t st);
+void launch_csr_fill(const FaceArrays& f, const int64_t* face_off, const int64_t* conn_off,
+                     const int32_t* in_count, int32_t* cursor, int n, int32_t* conn, const int32_t* pos, int nj,
+                     cudaStream_t st);
 }  // namespace mv
 
 namespace mv {
@@ -246,9 +243,11 @@ struct mv_context {
 namespace {
 constexpr size_t READBACK_BYTES = 1 << 20;
 
-__global__ void readback_kernel(const uint32_t* __restrict__ src, uint32_t* __restrict__ dst, int nwords) {
+// nwords words, in pieces of `piece` words that lie `stride` words apart
+__global__ void readback_kernel(const uint32_t* __restrict__ src, uint32_t* __restrict__ dst, int nwords,
+                                int piece, int64_t stride) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nwords; i += gridDim.x * blockDim.x)
-    dst[i] = src[i];
+    dst[i] = src[(i / piece) * stride + i % piece];
 }
 }  // namespace
 
@@ -302,19 +301,24 @@ T* P(DevBuf& b) {
 // It goes through a kernel into the context's mapped pinned buffer rather than a
 // cudaMemcpy: a copy would queue on the copy engine behind any bulk result copy that
 // another context has in flight, stalling this build until that copy ends.
-int readback(mv_context* ctx, void* dst, const void* src, size_t bytes, cudaStream_t st) {
+// `pieces` pieces of `bytes` bytes that lie `stride` bytes apart come back to back.
+int readback(mv_context* ctx, void* dst, const void* src, size_t bytes, cudaStream_t st, int pieces = 1,
+             size_t stride = 0) {
   if (bytes == 0) return MV_OK;
-  if (ctx->rb_dev && bytes % 4 == 0 && bytes <= READBACK_BYTES &&
+  if (ctx->rb_dev && bytes % 4 == 0 && stride % 4 == 0 && bytes * pieces <= READBACK_BYTES &&
       reinterpret_cast<uintptr_t>(src) % 4 == 0) {
-    const int nw = (int)(bytes / 4);
+    const int nw = (int)(bytes * pieces / 4);
     readback_kernel<<<std::min(64, (nw + 255) / 256), 256, 0, st>>>(
-        static_cast<const uint32_t*>(src), static_cast<uint32_t*>(ctx->rb_dev), nw);
+        static_cast<const uint32_t*>(src), static_cast<uint32_t*>(ctx->rb_dev), nw, (int)(bytes / 4),
+        (int64_t)(stride / 4));
     MV_CUDA(cudaGetLastError());
     MV_CUDA(cudaStreamSynchronize(st));
-    std::memcpy(dst, ctx->rb_host, bytes);
+    std::memcpy(dst, ctx->rb_host, bytes * pieces);
     return MV_OK;
   }
-  MV_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st));
+  for (int k = 0; k < pieces; k++)
+    MV_CUDA(cudaMemcpyAsync(static_cast<char*>(dst) + k * bytes, static_cast<const char*>(src) + k * stride, bytes,
+                            cudaMemcpyDeviceToHost, st));
   MV_CUDA(cudaStreamSynchronize(st));
   return MV_OK;
 }
@@ -674,11 +678,10 @@ int export_cells(mv_context* ctx, const Job& J, int64_t n, int flags, cudaStream
   (*launches)++;
   int64_t tot[5] = {0, 0, 0, 0, 0};
   if (n > 0) {
-    for (int k = 0; k < 5; k++) {
-      scan_i32_to_i64(cnt + k * N, n, off + k * (N + 1), P<long long>(W.scan_tmp), st);
-      MV_RB(&tot[k], off + k * (N + 1) + n, 8);
-    }
-    *launches += 15;
+    if (ensure(ctx, W.scan_tmp, 8 * 5 * scan_tmp_elems(n))) return MV_ERR_OOM;
+    *launches += scan_rows_i32_to_i64(cnt, n, 5, (int64_t)N, off, P<long long>(W.scan_tmp), st);
+    const int rb = readback(ctx, tot, off + n, 8, st, 5, 8 * (N + 1));
+    if (rb) return rb;
   } else {
     MV_CUDA(cudaMemsetAsync(off, 0, 8 * 5 * (N + 1), st));
   }
@@ -822,11 +825,11 @@ int build_device_impl(mv_context* ctx, const double* d_xyz, const uint8_t* d_mas
 
     // ---- generators + grid (replaces build_rtree, rtree_nn.rs:6-8) ----
     MV_CUDA(cudaEventRecord(ctx->ev[0], st));
-    launches = 13;  // prep, extent, cell index, 3 x 3 scan kernels, dense flags, scatter
+    launches = 3;  // prep, extent, scatter
     launch_prep(d_xyz, ni, s.dim, P<double>(W.gen), C->ext_keys, C->ext, &C->bad_input, st);
-    launch_grid_coarse(P<double>(W.gen), ni, s.G, s.anchor, s.ginv, P<int32_t>(W.cid),
-                       P<int32_t>(W.cell_count), P<int32_t>(W.cell_start), P<int32_t>(W.dflag),
-                       P<int32_t>(W.dprefix), s.dim, P<long long>(W.scan_tmp), st);
+    launches += launch_grid_coarse(P<double>(W.gen), ni, s.G, s.anchor, s.ginv, P<int32_t>(W.cid),
+                                   P<int32_t>(W.cell_count), P<int32_t>(W.cell_start), P<int32_t>(W.dflag),
+                                   P<int32_t>(W.dprefix), s.dim, P<long long>(W.scan_tmp), st);
     int32_t ndense = 0;
     MV_RB(&ndense, P<int32_t>(W.dprefix) + ncell, 4);
     if (ndense > 0) {
@@ -962,27 +965,30 @@ int build_device_impl(mv_context* ctx, const double* d_xyz, const uint8_t* d_mas
     if (e) return MV_ERR_OOM;
   }
   MV_CUDA(cudaEventRecord(ctx->ev[5], st));
-  scan_i32_to_i64(P<int32_t>(W.face_count), n, P<int64_t>(W.face_off), P<long long>(W.scan_tmp), st);
-  launches += 4;  // scan (3) + reorder
+  launches += 1 + scan_i32_to_i64(P<int32_t>(W.face_count), n, P<int64_t>(W.face_off),
+                                  P<long long>(W.scan_tmp), st);  // and the reordering
   FaceArrays stage{P<int32_t>(W.st_left), P<int32_t>(W.st_right), P<double>(W.st_area),
                    P<double>(W.st_cen), P<double>(W.st_nrm), P<uint8_t>(W.st_code)};
   FaceArrays fin{P<int32_t>(W.f_left), P<int32_t>(W.f_right), P<double>(W.f_area),
                  P<double>(W.f_cen), P<double>(W.f_nrm), P<uint8_t>(W.f_code)};
-  launch_reorder(stage, F, P<int64_t>(W.stage_off), P<int64_t>(W.face_off), fin, st);
+  const bool csr = o.face_mode == MV_FACES_OWNED;
+  if (csr) {
+    MV_CUDA(cudaMemsetAsync(W.in_count.p, 0, 4 * N, st));
+    MV_CUDA(cudaMemsetAsync(W.cursor.p, 0, 4 * N, st));
+  }
+  launch_reorder(stage, ni, P<int64_t>(W.stage_off), P<int64_t>(W.face_off), fin,
+                 csr ? P<int32_t>(W.in_count) : nullptr, nullptr, 0, st);
 
   // ---- Voronoi::finalize: cell -> face CSR (voronoi.rs:241-263) ----
   int64_t Cn = 0;
-  if (o.face_mode == MV_FACES_OWNED) {
-    MV_CUDA(cudaMemsetAsync(W.in_count.p, 0, 4 * N, st));
-    MV_CUDA(cudaMemsetAsync(W.cursor.p, 0, 4 * N, st));
-    launch_csr_counts(fin, F, P<int32_t>(W.face_count), ni, P<int32_t>(W.in_count),
-                      P<int32_t>(W.conn_count), st);
-    scan_i32_to_i64(P<int32_t>(W.conn_count), n, P<int64_t>(W.conn_off), P<long long>(W.scan_tmp), st);
+  if (csr) {
+    launches += 2 + launch_csr_offsets(P<int32_t>(W.face_count), P<int32_t>(W.in_count), n,
+                                       P<int32_t>(W.conn_count), P<int64_t>(W.conn_off),
+                                       P<long long>(W.scan_tmp), st);  // and fill, sort
     MV_RB(&Cn, P<int64_t>(W.conn_off) + n, 8);
     if (ensure(ctx, W.conn, 4 * (size_t)std::max<int64_t>(Cn, 1))) return MV_ERR_OOM;
-    launch_csr_fill(fin, F, P<int64_t>(W.face_off), P<int64_t>(W.conn_off), P<int32_t>(W.in_count),
-                    P<int32_t>(W.cursor), ni, P<int32_t>(W.conn), st);
-    launches += 7;  // in-count, conn-count, scan (3), fill, sort
+    launch_csr_fill(fin, P<int64_t>(W.face_off), P<int64_t>(W.conn_off), P<int32_t>(W.in_count),
+                    P<int32_t>(W.cursor), ni, P<int32_t>(W.conn), nullptr, 0, st);
   }
   MV_CUDA(cudaEventRecord(ctx->ev[6], st));
   MV_CUDA(cudaGetLastError());
@@ -1168,20 +1174,18 @@ int build_batch_device_impl(mv_context* ctx, const double* d_xyz, const uint8_t*
 
     // ---- generators + batch grid ----
     MV_CUDA(cudaEventRecord(ctx->ev[0], st));
-    launch_batch_grid(d_xyz, ni, d_pos, P<int32_t>(W.b_cbase), nj, P<BatchGrid>(W.b_grid), ncell,
-                      P<double>(W.gen), P<unsigned long long>(W.b_ext_keys), P<double>(W.b_ext),
-                      &C->bad_input, P<int32_t>(W.cid), P<int32_t>(W.cell_count),
-                      P<int32_t>(W.cell_start), P<int32_t>(W.dflag), P<int32_t>(W.dprefix),
-                      P<long long>(W.scan_tmp), st);
+    launches += launch_batch_grid(d_xyz, ni, d_pos, P<int32_t>(W.b_cbase), nj, P<BatchGrid>(W.b_grid), ncell,
+                                  P<double>(W.gen), P<unsigned long long>(W.b_ext_keys), P<double>(W.b_ext),
+                                  &C->bad_input, P<int32_t>(W.cid), P<int32_t>(W.cell_count),
+                                  P<int32_t>(W.cell_start), P<int32_t>(W.dflag), P<int32_t>(W.dprefix),
+                                  P<long long>(W.scan_tmp), st);
     MV_CUDA(launch_batch_sort(P<double>(W.gen), ni, d_pos, P<int32_t>(W.b_cbase), nj, P<BatchGrid>(W.b_grid),
                               ncell, P<int32_t>(W.cid), P<int32_t>(W.dflag), P<unsigned long long>(W.dkey_a),
                               P<unsigned long long>(W.dkey_b), P<int32_t>(W.dval_a), P<int32_t>(W.dval_b),
                               W.dsort_tmp.p, W.dsort_tmp.cap, P<double>(W.sx), P<double>(W.sy),
                               P<double>(W.sz), P<int32_t>(W.sid), P<uint32_t>(W.fkey),
                               P<int32_t>(W.cell_start), st));
-    // ext init / prep / finish, cell index, 2 x 3 scan kernels, dense flags, keys, sort,
-    // gather, starts
-    launches += 19;
+    launches += 8;  // keys, gather, the sort's passes, starts
 
     // ---- one Job per tessellation, addressing its slices ----
     for (int j = 0; j < nj; j++) {
@@ -1283,26 +1287,29 @@ int build_batch_device_impl(mv_context* ctx, const double* d_xyz, const uint8_t*
     if (e) return MV_ERR_OOM;
   }
   MV_CUDA(cudaEventRecord(ctx->ev[5], st));
-  scan_i32_to_i64(P<int32_t>(W.face_count), ntot, P<int64_t>(W.face_off), P<long long>(W.scan_tmp), st);
+  launches += 1 + scan_i32_to_i64(P<int32_t>(W.face_count), ntot, P<int64_t>(W.face_off),
+                                  P<long long>(W.scan_tmp), st);  // and the reordering
   FaceArrays stage{P<int32_t>(W.st_left), P<int32_t>(W.st_right), P<double>(W.st_area),
                    P<double>(W.st_cen), P<double>(W.st_nrm), P<uint8_t>(W.st_code)};
   FaceArrays fin{P<int32_t>(W.f_left), P<int32_t>(W.f_right), P<double>(W.f_area),
                  P<double>(W.f_cen), P<double>(W.f_nrm), P<uint8_t>(W.f_code)};
-  launch_reorder(stage, F, P<int64_t>(W.stage_off), P<int64_t>(W.face_off), fin, st);
-  launches += 4;
   int64_t Cn = 0;
   const bool owned = o.face_mode == MV_FACES_OWNED;
   if (owned) {
     MV_CUDA(cudaMemsetAsync(W.in_count.p, 0, 4 * N, st));
     MV_CUDA(cudaMemsetAsync(W.cursor.p, 0, 4 * N, st));
-    launch_batch_csr(fin, F, P<int64_t>(W.face_off), P<int32_t>(W.face_count), ni, d_pos, nj,
-                     P<int32_t>(W.in_count), P<int32_t>(W.conn_count), st);
-    scan_i32_to_i64(P<int32_t>(W.conn_count), ntot, P<int64_t>(W.conn_off), P<long long>(W.scan_tmp), st);
+  }
+  // faces carry the batch position of their left cell until the CSR is built
+  launch_reorder(stage, ni, P<int64_t>(W.stage_off), P<int64_t>(W.face_off), fin,
+                 owned ? P<int32_t>(W.in_count) : nullptr, d_pos, nj, st);
+  if (owned) {
+    launches += 2 + launch_csr_offsets(P<int32_t>(W.face_count), P<int32_t>(W.in_count), ntot,
+                                       P<int32_t>(W.conn_count), P<int64_t>(W.conn_off),
+                                       P<long long>(W.scan_tmp), st);  // and fill, sort
     MV_RB(&Cn, P<int64_t>(W.conn_off) + ntot, 8);
     if (ensure(ctx, W.conn, 4 * (size_t)std::max<int64_t>(Cn, 1))) return MV_ERR_OOM;
-    launch_batch_csr_fill(fin, F, P<int64_t>(W.face_off), P<int64_t>(W.conn_off), P<int32_t>(W.in_count),
-                          P<int32_t>(W.cursor), ni, d_pos, nj, P<int32_t>(W.conn), st);
-    launches += 7;
+    launch_csr_fill(fin, P<int64_t>(W.face_off), P<int64_t>(W.conn_off), P<int32_t>(W.in_count),
+                    P<int32_t>(W.cursor), ni, P<int32_t>(W.conn), d_pos, nj, st);
   }
   launch_batch_localize(fin, F, P<int64_t>(W.face_off), owned ? P<int64_t>(W.conn_off) : nullptr,
                         P<int32_t>(W.conn_count), P<int32_t>(W.conn), ni, d_pos, nj, P<int64_t>(W.b_fbase),

@@ -152,13 +152,22 @@ __global__ void dense_gather_kernel(const double* __restrict__ gen, int n,
 }
 
 // ------------------------------------------------------------------- scans --
-// Exclusive scan of int32 counts into int64 offsets, out[n] = total.
+// Exclusive scans of int32 counts into offsets, out[n] = total; blockIdx.y scans several
+// arrays of one length at once.  What bounds a scan here is launches (about 3 us each where
+// the arrays are small), so: up to SCAN_ONE counts one block does all (1,000 cells: 4 us,
+// where the three launches of reduce, scan of the sums and final took 11); up to SCAN_SUMS
+// tiles two launches, every final block adding up the sums before its own (a few KB out of
+// L2 each); only beyond, where that adding would grow with the square of the tiles, a third
+// launch that scans the sums.
 constexpr int SCAN_THREADS = 256;
 constexpr int SCAN_ITEMS = 16;
 constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
+constexpr int SCAN_ONE = 1024 * SCAN_ITEMS;
+constexpr int SCAN_SUMS = 2048;
 
+template <int THREADS>
 __device__ __forceinline__ long long block_excl_scan(long long v, long long* total) {
-  __shared__ long long wsum[SCAN_THREADS / 32];
+  __shared__ long long wsum[THREADS / 32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   long long x = v;
   for (int o = 1; o < 32; o <<= 1) {
@@ -168,59 +177,74 @@ __device__ __forceinline__ long long block_excl_scan(long long v, long long* tot
   if (lane == 31) wsum[w] = x;
   __syncthreads();
   if (w == 0) {
-    long long s = lane < SCAN_THREADS / 32 ? wsum[lane] : 0;
+    long long s = lane < THREADS / 32 ? wsum[lane] : 0;
     for (int o = 1; o < 32; o <<= 1) {
       long long y = __shfl_up_sync(0xffffffffu, s, o);
       if (lane >= o) s += y;
     }
-    if (lane < SCAN_THREADS / 32) wsum[lane] = s;
+    if (lane < THREADS / 32) wsum[lane] = s;
   }
   __syncthreads();
   long long wpre = w > 0 ? wsum[w - 1] : 0;
-  *total = wsum[SCAN_THREADS / 32 - 1];
+  *total = wsum[THREADS / 32 - 1];
   __syncthreads();
   return wpre + x - v;
 }
 
-template <class In>
-__global__ void scan_reduce_kernel(const In* __restrict__ in, int64_t n, long long* __restrict__ sums) {
+// What is scanned: in[k], or in[k] + add[k], which is then also kept in sum[k].
+struct ScanIn {
+  const int32_t* in;
+  const int32_t* add;
+  int32_t* sum;
+  int64_t stride;  // between the arrays of blockIdx.y
+};
+__device__ __forceinline__ int32_t scan_load(const ScanIn& a, int64_t k) {
+  int32_t v = a.in[a.stride * blockIdx.y + k];
+  if (a.add != nullptr) {
+    v += a.add[k];
+    a.sum[k] = v;
+  }
+  return v;
+}
+
+__global__ void scan_reduce_kernel(ScanIn a, int64_t n, long long* __restrict__ sums) {
   int64_t base = (int64_t)blockIdx.x * SCAN_TILE;
   long long s = 0;
   for (int i = 0; i < SCAN_ITEMS; i++) {
     int64_t k = base + (int64_t)i * SCAN_THREADS + threadIdx.x;
-    if (k < n) s += (long long)in[k];
+    if (k < n) s += scan_load(a, k);
   }
   long long tot;
-  block_excl_scan(s, &tot);
-  if (threadIdx.x == 0) sums[blockIdx.x] = tot;
+  block_excl_scan<SCAN_THREADS>(s, &tot);
+  if (threadIdx.x == 0) sums[(int64_t)gridDim.x * blockIdx.y + blockIdx.x] = tot;
 }
 
 __global__ void scan_sums_kernel(long long* sums, int nb) {
+  sums += (int64_t)nb * blockIdx.y;
   long long carry = 0;
   for (int base = 0; base < nb; base += SCAN_THREADS) {
     int k = base + threadIdx.x;
     long long v = k < nb ? sums[k] : 0;
     long long tot;
-    long long ex = block_excl_scan(v, &tot);
+    long long ex = block_excl_scan<SCAN_THREADS>(v, &tot);
     if (k < nb) sums[k] = carry + ex;
     carry += tot;
   }
 }
 
-template <class In, class Out>
-__global__ void scan_final_kernel(const In* __restrict__ in, int64_t n, const long long* __restrict__ sums,
-                                  Out* __restrict__ out) {
-  int64_t base = (int64_t)blockIdx.x * SCAN_TILE;
-  // each thread owns SCAN_ITEMS consecutive items
-  long long v[SCAN_ITEMS];
+// One tile: each thread owns SCAN_ITEMS consecutive counts; `before` is added to all.
+template <int THREADS, class Out>
+__device__ __forceinline__ void scan_tile(const ScanIn& a, int64_t base, int64_t n, long long before,
+                                          Out* __restrict__ out) {
+  int32_t v[SCAN_ITEMS];
   long long s = 0;
   for (int i = 0; i < SCAN_ITEMS; i++) {
     int64_t k = base + (int64_t)threadIdx.x * SCAN_ITEMS + i;
-    v[i] = k < n ? (long long)in[k] : 0;
+    v[i] = k < n ? scan_load(a, k) : 0;
     s += v[i];
   }
   long long tot;
-  long long ex = block_excl_scan(s, &tot) + sums[blockIdx.x];
+  long long ex = block_excl_scan<THREADS>(s, &tot) + before;
   for (int i = 0; i < SCAN_ITEMS; i++) {
     int64_t k = base + (int64_t)threadIdx.x * SCAN_ITEMS + i;
     if (k < n) out[k] = (Out)ex;
@@ -229,76 +253,146 @@ __global__ void scan_final_kernel(const In* __restrict__ in, int64_t n, const lo
   }
 }
 
+template <class Out>
+__global__ void scan_final_kernel(ScanIn a, int64_t n, const long long* __restrict__ sums, bool scanned,
+                                  Out* __restrict__ out, int64_t out_stride) {
+  sums += (int64_t)gridDim.x * blockIdx.y;
+  long long before = 0;
+  if (scanned) {
+    before = sums[blockIdx.x];
+  } else {
+    for (int k = threadIdx.x; k < (int)blockIdx.x; k += SCAN_THREADS) before += sums[k];
+    long long mine = before;
+    block_excl_scan<SCAN_THREADS>(mine, &before);
+  }
+  scan_tile<SCAN_THREADS>(a, (int64_t)blockIdx.x * SCAN_TILE, n, before, out + out_stride * blockIdx.y);
+}
+
+template <class Out>
+__global__ void __launch_bounds__(1024) scan_one_kernel(ScanIn a, int64_t n, Out* __restrict__ out, int64_t out_stride) {
+  scan_tile<1024>(a, 0, n, 0, out + out_stride * blockIdx.y);
+}
+
 // --------------------------------------------------------------- faces/CSR --
 
-// staging slot -> final position: faces grouped by left cell in cell order, inside a
-// cell in clipping-plane order (flatten!, voronoi.rs:226)
-__global__ void reorder_faces_kernel(FaceArrays st, int64_t F, const int64_t* __restrict__ stage_off,
-                                     const int64_t* __restrict__ face_off, FaceArrays out) {
-  int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= F) return;
-  int left = st.left[q];
-  int64_t f = face_off[left] + (q - stage_off[left]);
-  out.left[f] = left;
-  out.right[f] = st.right[q];
-  out.area[f] = st.area[q];
-  for (int i = 0; i < 3; i++) {
-    out.centroid[3 * f + i] = st.centroid[3 * q + i];
-    out.normal[3 * f + i] = st.normal[3 * q + i];
+__device__ __forceinline__ int batch_find(const int32_t* __restrict__ base, int nj, int64_t v);
+
+// Lanes that share a cell in the kernels below: a cell owns about 8 faces (3-D).
+constexpr int FACE_LANES = 8;
+
+// Staging slots -> final positions: faces grouped by left cell in cell order, inside a
+// cell in clipping-plane order (flatten!, voronoi.rs:226).  Bound by memory: 69 bytes of a
+// face read and written once.  Cells come out of the pipeline in grid order, so a cell's
+// faces lie together on both sides but neighbouring cells only on the written side: eight
+// lanes copy a cell, so that the writes of a warp are one run and the scattered side is
+// read, where a sector that is used in part costs less than one written in part.  16.5 M
+// faces: 1.27 ms with a thread per face in staging order, and 0.09 ms more for the counts.
+// Also counts the faces linked to their right cell (voronoi.rs:248-250: internal,
+// unshifted faces; in_count null: not wanted); a batch's right indices are local to
+// their tessellation (pos, nj).
+__global__ void reorder_faces_kernel(FaceArrays st, int n, const int64_t* __restrict__ stage_off,
+                                     const int64_t* __restrict__ face_off, FaceArrays out,
+                                     int32_t* __restrict__ in_count, const int32_t* __restrict__ pos, int nj) {
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int g = (int)(t % FACE_LANES);
+  const int64_t k = t / FACE_LANES;
+  if (k >= n) return;
+  const int64_t f0 = face_off[k];
+  const int m = (int)(face_off[k + 1] - f0);
+  if (m == 0) return;
+  const int64_t q0 = stage_off[k];
+  const int first = pos != nullptr && in_count != nullptr ? pos[batch_find(pos, nj, k)] : 0;
+  for (int i = g; i < m; i += FACE_LANES) {
+    const int32_t r = st.right[q0 + i];
+    const uint8_t code = st.code[q0 + i];
+    const double area = st.area[q0 + i];
+    out.left[f0 + i] = (int32_t)k;
+    out.right[f0 + i] = r;
+    out.area[f0 + i] = area;
+    out.code[f0 + i] = code;
+    if (in_count != nullptr && r >= 0 && code == 13) atomicAdd(in_count + first + r, 1);
   }
-  out.code[f] = st.code[q];
-}
-
-// faces linked to their right cell (voronoi.rs:248-250: internal, unshifted faces)
-__global__ void in_count_kernel(const int32_t* __restrict__ right, const uint8_t* __restrict__ code,
-                                int64_t F, int32_t* __restrict__ in_count) {
-  int64_t f = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= F) return;
-  int r = right[f];
-  if (r >= 0 && code[f] == 13) atomicAdd(in_count + r, 1);
-}
-
-__global__ void conn_count_kernel(const int32_t* __restrict__ face_count,
-                                  const int32_t* __restrict__ in_count, int n,
-                                  int32_t* __restrict__ conn_count) {
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < n) conn_count[k] = face_count[k] + in_count[k];
+  const double* c = st.centroid + 3 * q0;
+  const double* v = st.normal + 3 * q0;
+  double* oc = out.centroid + 3 * f0;
+  double* ov = out.normal + 3 * f0;
+  // four loads of each in flight per lane: 3 m is 24 where a cell owns 8 faces
+  for (int b = g; b < 3 * m; b += 4 * FACE_LANES) {
+    double x[4], y[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+      if (b + u * FACE_LANES < 3 * m) x[u] = c[b + u * FACE_LANES], y[u] = v[b + u * FACE_LANES];
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+      if (b + u * FACE_LANES < 3 * m) oc[b + u * FACE_LANES] = x[u], ov[b + u * FACE_LANES] = y[u];
+  }
 }
 
 // A cell's connections are its incoming faces (all from lower-indexed cells, so with
 // smaller face indices) followed by its own faces in order.
-__global__ void conn_fill_kernel(const int32_t* __restrict__ left, const int32_t* __restrict__ right,
-                                 const uint8_t* __restrict__ code, int64_t F,
-                                 const int64_t* __restrict__ face_off,
-                                 const int64_t* __restrict__ conn_off,
+__global__ void conn_fill_kernel(const int32_t* __restrict__ right, const uint8_t* __restrict__ code, int n,
+                                 const int64_t* __restrict__ face_off, const int64_t* __restrict__ conn_off,
                                  const int32_t* __restrict__ in_count, int32_t* __restrict__ cursor,
-                                 int32_t* __restrict__ conn) {
-  int64_t f = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= F) return;
-  int l = left[f];
-  conn[conn_off[l] + in_count[l] + (f - face_off[l])] = (int32_t)f;
-  int r = right[f];
-  if (r >= 0 && code[f] == 13) {
-    int slot = atomicAdd(cursor + r, 1);
-    conn[conn_off[r] + slot] = (int32_t)f;
+                                 int32_t* __restrict__ conn, const int32_t* __restrict__ pos, int nj) {
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int g = (int)(t % FACE_LANES);
+  const int64_t k = t / FACE_LANES;
+  if (k >= n) return;
+  const int64_t f0 = face_off[k], f1 = face_off[k + 1];
+  if (f0 == f1) return;
+  const int first = pos != nullptr ? pos[batch_find(pos, nj, k)] : 0;
+  int32_t* own = conn + conn_off[k] + in_count[k];
+  for (int64_t f = f0 + g; f < f1; f += FACE_LANES) {
+    own[f - f0] = (int32_t)f;
+    const int32_t r = right[f];
+    if (r >= 0 && code[f] == 13) conn[conn_off[first + r] + atomicAdd(cursor + first + r, 1)] = (int32_t)f;
   }
 }
 
+// The incoming faces in ascending order, whatever order the atomics gave.  Eight lanes rank
+// a cell's faces against one another (a face's place is the number of smaller ones), up to
+// four a lane; a cell with more is sorted by insertion, which was every cell's way before:
+// 24 us for 1,000 cells, one thread a cell, all of it the latency of dependent accesses.
 __global__ void conn_sort_kernel(const int64_t* __restrict__ conn_off,
                                  const int32_t* __restrict__ in_count, int n,
                                  int32_t* __restrict__ conn) {
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int g = (int)(t % FACE_LANES);
+  const int64_t k = t / FACE_LANES;
+  const unsigned group = 0xffu << (threadIdx.x & 24);  // the lanes of this cell
   if (k >= n) return;
   int32_t* a = conn + conn_off[k];
-  int m = in_count[k];
-  for (int i = 1; i < m; i++) {
-    int32_t v = a[i];
-    int j = i - 1;
-    while (j >= 0 && a[j] > v) {
-      a[j + 1] = a[j];
-      j--;
+  const int m = in_count[k];
+  if (m <= 4 * FACE_LANES) {
+    int32_t v[4];
+    int rank[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      v[u] = g + u * FACE_LANES < m ? a[g + u * FACE_LANES] : 0x7fffffff;
+      rank[u] = 0;
     }
-    a[j + 1] = v;
+#pragma unroll
+    for (int w = 0; w < 4; w++) {
+      if (w * FACE_LANES >= m) break;
+      for (int j = 0; j < FACE_LANES; j++) {
+        const int32_t o = __shfl_sync(group, v[w], j, FACE_LANES);
+#pragma unroll
+        for (int u = 0; u < 4; u++) rank[u] += o < v[u];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+      if (g + u * FACE_LANES < m) a[rank[u]] = v[u];
+  } else if (g == 0) {
+    for (int i = 1; i < m; i++) {
+      int32_t v = a[i];
+      int j = i - 1;
+      while (j >= 0 && a[j] > v) {
+        a[j + 1] = a[j];
+        j--;
+      }
+      a[j + 1] = v;
+    }
   }
 }
 
@@ -441,36 +535,6 @@ __global__ void batch_local_starts_kernel(int32_t* __restrict__ start, int64_t n
   start[c] -= pos[batch_find(cbase, nj, c)];
 }
 
-// Voronoi::finalize over a batch: faces carry the batch position of their left cell
-// until the CSR is built; right indices are local to the tessellation
-__global__ void batch_in_count_kernel(const int32_t* __restrict__ left, const int32_t* __restrict__ right,
-                                      const uint8_t* __restrict__ code, int64_t F,
-                                      const int32_t* __restrict__ pos, int nj,
-                                      int32_t* __restrict__ in_count) {
-  const int64_t f = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= F) return;
-  const int r = right[f];
-  if (r >= 0 && code[f] == 13) atomicAdd(in_count + r + pos[batch_find(pos, nj, left[f])], 1);
-}
-
-__global__ void batch_conn_fill_kernel(const int32_t* __restrict__ left, const int32_t* __restrict__ right,
-                                       const uint8_t* __restrict__ code, const int64_t* __restrict__ face_off,
-                                       const int64_t* __restrict__ conn_off,
-                                       const int32_t* __restrict__ in_count, int32_t* __restrict__ cursor,
-                                       int64_t F, const int32_t* __restrict__ pos, int nj,
-                                       int32_t* __restrict__ conn) {
-  const int64_t f = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= F) return;
-  const int l = left[f];
-  conn[conn_off[l] + in_count[l] + (f - face_off[l])] = (int32_t)f;
-  const int r = right[f];
-  if (r >= 0 && code[f] == 13) {
-    const int rg = r + pos[batch_find(pos, nj, l)];
-    const int slot = atomicAdd(cursor + rg, 1);
-    conn[conn_off[rg] + slot] = (int32_t)f;
-  }
-}
-
 // first face and first connection of each tessellation (j = nj: the totals)
 __global__ void batch_bases_kernel(const int64_t* __restrict__ face_off, const int64_t* __restrict__ conn_off,
                                    const int32_t* __restrict__ pos, int nj, int64_t* __restrict__ fbase,
@@ -516,25 +580,40 @@ void launch_grid(const double* gen, int n, const int G[3], const double a[3], co
                  int32_t* cid, int32_t* count, int32_t* start, int32_t* fill, double* sx, double* sy,
                  double* sz, int32_t* sid, long long* scan_tmp, cudaStream_t st);
 
-template <class In, class Out>
-static void scan_impl(const In* in, int64_t n, Out* out, long long* tmp, cudaStream_t st) {
-  if (n <= 0) {
-    cudaMemsetAsync(out, 0, sizeof(Out), st);
-    return;
-  }
-  int nb = (int)((n + SCAN_TILE - 1) / SCAN_TILE);
-  scan_reduce_kernel<In><<<nb, SCAN_THREADS, 0, st>>>(in, n, tmp);
-  scan_sums_kernel<<<1, SCAN_THREADS, 0, st>>>(tmp, nb);
-  scan_final_kernel<In, Out><<<nb, SCAN_THREADS, 0, st>>>(in, n, tmp, out);
-}
-
 size_t scan_tmp_elems(int64_t n) { return (size_t)((n + SCAN_TILE - 1) / SCAN_TILE) + 1; }
 
-void scan_i32_to_i32(const int32_t* in, int64_t n, int32_t* out, long long* tmp, cudaStream_t st) {
-  scan_impl<int32_t, int32_t>(in, n, out, tmp, st);
+// rows scans of n counts each; tmp holds rows * scan_tmp_elems(n).  Returns the launches.
+template <class Out>
+static int scan_impl(const ScanIn& a, int64_t n, int rows, Out* out, int64_t out_stride, long long* tmp,
+                     cudaStream_t st) {
+  if (n <= 0) {
+    for (int r = 0; r < rows; r++) cudaMemsetAsync(out + r * out_stride, 0, sizeof(Out), st);
+    return 0;
+  }
+  if (n <= SCAN_ONE) {
+    scan_one_kernel<Out><<<dim3(1, rows), 1024, 0, st>>>(a, n, out, out_stride);
+    return 1;
+  }
+  const int nb = (int)((n + SCAN_TILE - 1) / SCAN_TILE);
+  const bool scanned = nb > SCAN_SUMS;
+  ScanIn final = a;
+  if (a.add) final.in = a.sum, final.add = nullptr;  // the sums are there by then
+  scan_reduce_kernel<<<dim3(nb, rows), SCAN_THREADS, 0, st>>>(a, n, tmp);
+  if (scanned) scan_sums_kernel<<<dim3(1, rows), SCAN_THREADS, 0, st>>>(tmp, nb);
+  scan_final_kernel<Out><<<dim3(nb, rows), SCAN_THREADS, 0, st>>>(final, n, tmp, scanned, out, out_stride);
+  return 2 + scanned;
 }
-void scan_i32_to_i64(const int32_t* in, int64_t n, int64_t* out, long long* tmp, cudaStream_t st) {
-  scan_impl<int32_t, int64_t>(in, n, out, tmp, st);
+
+int scan_i32_to_i32(const int32_t* in, int64_t n, int32_t* out, long long* tmp, cudaStream_t st) {
+  return scan_impl<int32_t>({in, nullptr, nullptr, 0}, n, 1, out, 0, tmp, st);
+}
+int scan_i32_to_i64(const int32_t* in, int64_t n, int64_t* out, long long* tmp, cudaStream_t st) {
+  return scan_impl<int64_t>({in, nullptr, nullptr, 0}, n, 1, out, 0, tmp, st);
+}
+// `rows` arrays of n counts, `stride` apart, into offsets n + 1 apart
+int scan_rows_i32_to_i64(const int32_t* in, int64_t n, int rows, int64_t stride, int64_t* out, long long* tmp,
+                         cudaStream_t st) {
+  return scan_impl<int64_t>({in, nullptr, nullptr, stride}, n, rows, out, n + 1, tmp, st);
 }
 
 void launch_grid(const double* gen, int n, const int G[3], const double a[3], const double inv[3],
@@ -551,8 +630,8 @@ void launch_grid(const double* gen, int n, const int G[3], const double a[3], co
 
 // First half of the two-level grid: coarse cell index, counts, starts and the dense
 // cells (flags and their running count).  The host reads the number of dense cells,
-// then calls launch_grid_dense (or scatters coarse-only).
-void launch_grid_coarse(const double* gen, int n, const int G[3], const double a[3],
+// then calls launch_grid_dense (or scatters coarse-only).  Returns the launches.
+int launch_grid_coarse(const double* gen, int n, const int G[3], const double a[3],
                         const double inv[3], int32_t* cid, int32_t* count, int32_t* start,
                         int32_t* dflag, int32_t* dprefix, int dim, long long* scan_tmp, cudaStream_t st) {
   GridParams gp;
@@ -560,9 +639,9 @@ void launch_grid_coarse(const double* gen, int n, const int G[3], const double a
   gp.dim = dim;
   const int64_t ncell = (int64_t)G[0] * G[1] * G[2];
   if (n > 0) cell_index_kernel<<<nblk(n, 256), 256, 0, st>>>(gen, n, gp, cid, count);
-  scan_i32_to_i32(count, ncell, start, scan_tmp, st);
+  int launches = 2 + scan_i32_to_i32(count, ncell, start, scan_tmp, st);
   dense_flag_kernel<<<nblk(ncell, 256), 256, 0, st>>>(count, ncell, dflag);
-  scan_i32_to_i32(dflag, ncell, dprefix, scan_tmp, st);
+  return launches + scan_i32_to_i32(dflag, ncell, dprefix, scan_tmp, st);
 }
 
 // Scratch bytes of launch_grid_dense's radix sort.
@@ -603,37 +682,41 @@ void launch_scatter(const double* gen, int n, const int32_t* cid, const int32_t*
   if (n > 0) scatter_kernel<<<nblk(n, 256), 256, 0, st>>>(gen, n, cid, start, fill, sx, sy, sz, sid);
 }
 
-void launch_reorder(const FaceArrays& stage, int64_t F, const int64_t* stage_off,
-                    const int64_t* face_off, const FaceArrays& out, cudaStream_t st) {
-  if (F > 0) reorder_faces_kernel<<<nblk(F, 256), 256, 0, st>>>(stage, F, stage_off, face_off, out);
+void launch_reorder(const FaceArrays& stage, int n, const int64_t* stage_off, const int64_t* face_off,
+                    const FaceArrays& out, int32_t* in_count, const int32_t* pos, int nj, cudaStream_t st) {
+  if (n > 0)
+    reorder_faces_kernel<<<nblk((int64_t)FACE_LANES * n, 256), 256, 0, st>>>(stage, n, stage_off, face_off, out,
+                                                                             in_count, pos, nj);
 }
 
-void launch_csr_counts(const FaceArrays& f, int64_t F, const int32_t* face_count, int n,
-                       int32_t* in_count, int32_t* conn_count, cudaStream_t st) {
-  if (F > 0) in_count_kernel<<<nblk(F, 256), 256, 0, st>>>(f.right, f.code, F, in_count);
-  if (n > 0) conn_count_kernel<<<nblk(n, 256), 256, 0, st>>>(face_count, in_count, n, conn_count);
+// conn_count[k] = own + incoming faces of cell k, conn_off = their scan.  Returns the launches.
+int launch_csr_offsets(const int32_t* face_count, const int32_t* in_count, int64_t n, int32_t* conn_count,
+                       int64_t* conn_off, long long* scan_tmp, cudaStream_t st) {
+  return scan_impl<int64_t>({face_count, in_count, conn_count, 0}, n, 1, conn_off, 0, scan_tmp, st);
 }
 
-void launch_csr_fill(const FaceArrays& f, int64_t F, const int64_t* face_off, const int64_t* conn_off,
-                     const int32_t* in_count, int32_t* cursor, int n, int32_t* conn, cudaStream_t st) {
-  if (F > 0)
-    conn_fill_kernel<<<nblk(F, 256), 256, 0, st>>>(f.left, f.right, f.code, F, face_off, conn_off,
-                                                   in_count, cursor, conn);
-  if (n > 0) conn_sort_kernel<<<nblk(n, 256), 256, 0, st>>>(conn_off, in_count, n, conn);
+void launch_csr_fill(const FaceArrays& f, const int64_t* face_off, const int64_t* conn_off,
+                     const int32_t* in_count, int32_t* cursor, int n, int32_t* conn, const int32_t* pos, int nj,
+                     cudaStream_t st) {
+  if (n <= 0) return;
+  const int nb = nblk((int64_t)FACE_LANES * n, 256);
+  conn_fill_kernel<<<nb, 256, 0, st>>>(f.right, f.code, n, face_off, conn_off, in_count, cursor, conn, pos, nj);
+  conn_sort_kernel<<<nb, 256, 0, st>>>(conn_off, in_count, n, conn);
 }
 
 // ------------------------------------------------------------ batch launchers --
-void launch_batch_grid(const double* xyz, int n, const int32_t* pos, const int32_t* cbase, int nj,
-                       const BatchGrid* bg, int64_t ncell, double* gen, unsigned long long* ext_keys,
-                       double* ext, int* bad, int32_t* cid, int32_t* count, int32_t* start,
-                       int32_t* dflag, int32_t* dprefix, long long* scan_tmp, cudaStream_t st) {
+// Returns the launches.
+int launch_batch_grid(const double* xyz, int n, const int32_t* pos, const int32_t* cbase, int nj,
+                      const BatchGrid* bg, int64_t ncell, double* gen, unsigned long long* ext_keys,
+                      double* ext, int* bad, int32_t* cid, int32_t* count, int32_t* start,
+                      int32_t* dflag, int32_t* dprefix, long long* scan_tmp, cudaStream_t st) {
   batch_ext_init_kernel<<<nblk(6 * (int64_t)nj, 256), 256, 0, st>>>(ext_keys, nj);
   if (n > 0) batch_prep_kernel<<<nblk(n, 256), 256, 0, st>>>(xyz, n, pos, nj, bg, gen, ext_keys, bad);
   batch_ext_finish_kernel<<<nblk(6 * (int64_t)nj, 256), 256, 0, st>>>(ext_keys, ext, nj);
   if (n > 0) batch_cell_index_kernel<<<nblk(n, 256), 256, 0, st>>>(gen, n, pos, nj, bg, cid, count);
-  scan_i32_to_i32(count, ncell, start, scan_tmp, st);
+  const int launches = 5 + scan_i32_to_i32(count, ncell, start, scan_tmp, st);
   dense_flag_kernel<<<nblk(ncell, 256), 256, 0, st>>>(count, ncell, dflag);
-  scan_i32_to_i32(dflag, ncell, dprefix, scan_tmp, st);
+  return launches + scan_i32_to_i32(dflag, ncell, dprefix, scan_tmp, st);
 }
 
 size_t batch_sort_bytes(int n, int64_t ncell) { return grid_dense_sort_bytes(n, ncell); }
@@ -654,23 +737,6 @@ cudaError_t launch_batch_sort(const double* gen, int n, const int32_t* pos, cons
   }
   batch_local_starts_kernel<<<nblk(ncell, 256), 256, 0, st>>>(start, ncell, cbase, pos, nj);
   return cudaGetLastError();
-}
-
-void launch_batch_csr(const FaceArrays& f, int64_t F, const int64_t* face_off, const int32_t* face_count,
-                      int n, const int32_t* pos, int nj, int32_t* in_count, int32_t* conn_count,
-                      cudaStream_t st) {
-  if (F > 0)
-    batch_in_count_kernel<<<nblk(F, 256), 256, 0, st>>>(f.left, f.right, f.code, F, pos, nj, in_count);
-  if (n > 0) conn_count_kernel<<<nblk(n, 256), 256, 0, st>>>(face_count, in_count, n, conn_count);
-}
-
-void launch_batch_csr_fill(const FaceArrays& f, int64_t F, const int64_t* face_off, const int64_t* conn_off,
-                           const int32_t* in_count, int32_t* cursor, int n, const int32_t* pos, int nj,
-                           int32_t* conn, cudaStream_t st) {
-  if (F > 0)
-    batch_conn_fill_kernel<<<nblk(F, 256), 256, 0, st>>>(f.left, f.right, f.code, face_off, conn_off,
-                                                         in_count, cursor, F, pos, nj, conn);
-  if (n > 0) conn_sort_kernel<<<nblk(n, 256), 256, 0, st>>>(conn_off, in_count, n, conn);
 }
 
 void launch_batch_localize(FaceArrays& f, int64_t F, const int64_t* face_off, int64_t* conn_off,

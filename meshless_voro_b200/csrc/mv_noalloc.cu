@@ -39,13 +39,14 @@ void launch_prep(const double* xyz, int n, int dim, double* gen, unsigned long l
 void launch_grid(const double* gen, int n, const int G[3], const double a[3], const double inv[3],
                  int32_t* cid, int32_t* count, int32_t* start, int32_t* fill, double* sx, double* sy,
                  double* sz, int32_t* sid, long long* scan_tmp, cudaStream_t st);
-void scan_i32_to_i64(const int32_t* in, int64_t n, int64_t* out, long long* tmp, cudaStream_t st);
-void launch_reorder(const FaceArrays& stage, int64_t F, const int64_t* stage_off,
-                    const int64_t* face_off, const FaceArrays& out, cudaStream_t st);
-void launch_csr_counts(const FaceArrays& f, int64_t F, const int32_t* face_count, int n,
-                       int32_t* in_count, int32_t* conn_count, cudaStream_t st);
-void launch_csr_fill(const FaceArrays& f, int64_t F, const int64_t* face_off, const int64_t* conn_off,
-                     const int32_t* in_count, int32_t* cursor, int n, int32_t* conn, cudaStream_t st);
+int scan_i32_to_i64(const int32_t* in, int64_t n, int64_t* out, long long* tmp, cudaStream_t st);
+void launch_reorder(const FaceArrays& stage, int n, const int64_t* stage_off, const int64_t* face_off,
+                    const FaceArrays& out, int32_t* in_count, const int32_t* pos, int nj, cudaStream_t st);
+int launch_csr_offsets(const int32_t* face_count, const int32_t* in_count, int64_t n, int32_t* conn_count,
+                       int64_t* conn_off, long long* scan_tmp, cudaStream_t st);
+void launch_csr_fill(const FaceArrays& f, const int64_t* face_off, const int64_t* conn_off,
+                     const int32_t* in_count, int32_t* cursor, int n, int32_t* conn, const int32_t* pos, int nj,
+                     cudaStream_t st);
 }  // namespace mv
 
 using namespace mv;
@@ -294,20 +295,22 @@ extern "C" int mv_voronoi_build_noalloc(const double* d_generators, const uint8_
                    at<double>(B, O_STCEN), at<double>(B, O_STNRM), at<uint8_t>(B, O_STCODE)};
   FaceArrays fin{out->face_left, out->face_right, out->face_area,
                  out->face_centroid, out->face_normal, out->face_shift_code};
-  launch_reorder(stage, F, at<int64_t>(B, O_STOFF), at<int64_t>(B, O_FOFF), fin, st);
   if (csr) {
     NA_CUDA(cudaMemsetAsync(B + O_INCNT, 0, 4 * n, st));
     NA_CUDA(cudaMemsetAsync(B + O_CURSOR, 0, 4 * n, st));
-    launch_csr_counts(fin, F, at<int32_t>(B, O_FCOUNT), ni, at<int32_t>(B, O_INCNT),
-                      out->cell_face_count, st);
-    scan_i32_to_i64(out->cell_face_count, n, at<int64_t>(B, O_CONNOFF), at<long long>(B, O_SCAN), st);
+  }
+  launch_reorder(stage, ni, at<int64_t>(B, O_STOFF), at<int64_t>(B, O_FOFF), fin,
+                 csr ? at<int32_t>(B, O_INCNT) : nullptr, nullptr, 0, st);
+  if (csr) {
+    launch_csr_offsets(at<int32_t>(B, O_FCOUNT), at<int32_t>(B, O_INCNT), n, out->cell_face_count,
+                       at<int64_t>(B, O_CONNOFF), at<long long>(B, O_SCAN), st);
     int64_t Cn = 0;
     NA_CUDA(cudaMemcpyAsync(&Cn, at<int64_t>(B, O_CONNOFF) + n, 8, cudaMemcpyDeviceToHost, st));
     NA_CUDA(cudaStreamSynchronize(st));
     out->n_connections = Cn;
     if (Cn > connection_capacity) return MV_ERR_CAPACITY;
-    launch_csr_fill(fin, F, at<int64_t>(B, O_FOFF), at<int64_t>(B, O_CONNOFF), at<int32_t>(B, O_INCNT),
-                    at<int32_t>(B, O_CURSOR), ni, out->cell_face_connections, st);
+    launch_csr_fill(fin, at<int64_t>(B, O_FOFF), at<int64_t>(B, O_CONNOFF), at<int32_t>(B, O_INCNT),
+                    at<int32_t>(B, O_CURSOR), ni, out->cell_face_connections, nullptr, 0, st);
     NA_CUDA(cudaMemcpyAsync(out->cell_face_offset, at<int64_t>(B, O_CONNOFF), 8 * n,
                             cudaMemcpyDeviceToDevice, st));
   }
