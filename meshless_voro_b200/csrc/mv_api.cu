@@ -57,8 +57,8 @@ int64_t stage_record_words(int np, int nv);
 void launch_prep(const double* xyz, int n, int dim, double* gen, unsigned long long* ext_keys,
                  double* ext, int* bad, cudaStream_t st);
 int launch_grid_coarse(const double* gen, int n, const int G[3], const double a[3],
-                        const double inv[3], int32_t* cid, int32_t* count, int32_t* start,
-                        int32_t* dflag, int32_t* dprefix, int dim, long long* scan_tmp, cudaStream_t st);
+                       const double inv[3], int32_t* cid, int32_t* count, int32_t* start,
+                       int32_t* dflag, int32_t* dprefix, int dim, long long* scan_tmp, cudaStream_t st);
 size_t grid_dense_sort_bytes(int n, int64_t ncell);
 int launch_batch_grid(const double* xyz, int n, const int32_t* pos, const int32_t* cbase, int nj,
                        const BatchGrid* bg, int64_t ncell, double* gen, unsigned long long* ext_keys,
@@ -69,6 +69,7 @@ cudaError_t launch_batch_sort(const double* gen, int n, const int32_t* pos, cons
                               unsigned long long* key_a, unsigned long long* key_b, int32_t* val_a,
                               int32_t* val_b, void* sort_tmp, size_t sort_bytes, double* sx, double* sy,
                               double* sz, int32_t* sid, uint32_t* fkey, int32_t* start, cudaStream_t st);
+void launch_batch_levels(Job* jobs, const int32_t* dprefix, const int32_t* cbase, int nj, cudaStream_t st);
 void launch_batch_localize(FaceArrays& f, int64_t F, const int64_t* face_off, int64_t* conn_off,
                            const int32_t* conn_count, int32_t* conn, int n, const int32_t* pos, int nj,
                            int64_t* fbase, int64_t* cbase_conn, cudaStream_t st);
@@ -1231,6 +1232,8 @@ int build_batch_device_impl(mv_context* ctx, const double* d_xyz, const uint8_t*
       J.id_base = (int32_t)pb;
     }
     MV_CUDA(cudaMemcpyAsync(W.b_jobs.p, JJ.data(), sizeof(Job) * (size_t)nj, cudaMemcpyHostToDevice, st));
+    launch_batch_levels(P<Job>(W.b_jobs), P<int32_t>(W.dprefix), P<int32_t>(W.b_cbase), nj, st);
+    launches++;
     // the template Job: shared fields (counters, staging, queues) and the batch's size
     Job J0 = JJ[0];
     J0.n = ni;

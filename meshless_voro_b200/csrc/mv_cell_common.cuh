@@ -208,15 +208,58 @@ struct CellCount {
 // ------------------------------------------------------------- neighbour shell --
 // First position in [a, b) whose dense-cell key is >= k (the keys of a dense cell are
 // sorted).
-__device__ __forceinline__ int32_t fkey_lower_bound(const Job& J, int32_t a, int32_t b, uint32_t k) {
-  while (a < b) {
-    const int32_t m = (a + b) >> 1;
-    if (__ldg(J.fkey + m) < k)
-      a = m + 1;
-    else
-      b = m;
+// The generators of a dense cell, [cs, ce), searched by a whole warp, a key pair per lane:
+// lane l holds the key of every step-th generator, so that a search finds its 32nd of the
+// cell by shuffles and only the rest by dependent loads, the pair's two searches side by
+// side.  (Cells of 1,000 to 40,000 generators: 5 to 10 loads in a row where two searches
+// one after the other took 20 to 30, a third of the time of a shell in a dense cell.)
+struct DenseSearch {
+  int32_t cs, ce, step;
+  uint32_t pivot;
+};
+__device__ __forceinline__ DenseSearch dense_search(const Job& J, int32_t cs, int32_t ce, int lane) {
+  DenseSearch s;
+  s.cs = cs, s.ce = ce;
+  s.step = (int32_t)((uint32_t)(ce - cs + 31) >> 5);
+  const int64_t at = (int64_t)cs + (int64_t)lane * s.step;
+  s.pivot = at < ce ? __ldg(J.fkey + at) : 0xffffffffu;
+  return s;
+}
+// First position with a key >= k; keys are below 2^32 - 1.  All lanes call it together.
+__device__ __forceinline__ void dense_bounds(const Job& J, const DenseSearch& s, uint32_t k0, uint32_t k1,
+                                             int32_t* p0, int32_t* p1) {
+  int n0 = 0, n1 = 0;  // pivots below the keys
+#pragma unroll
+  for (int b = 16; b > 0; b >>= 1) {
+    if (__shfl_sync(FULL, s.pivot, n0 + b - 1) < k0) n0 += b;
+    if (__shfl_sync(FULL, s.pivot, n1 + b - 1) < k1) n1 += b;
   }
-  return a;
+  const uint32_t last = __shfl_sync(FULL, s.pivot, 31);
+  n0 += n0 == 31 && last < k0;
+  n1 += n1 == 31 && last < k1;
+  // the answer lies past pivot n - 1 and at or before pivot n (no pivot below: at cs)
+  int32_t a0 = n0 > 0 ? s.cs + (n0 - 1) * s.step + 1 : s.cs, b0 = min(s.ce, s.cs + n0 * s.step);
+  int32_t a1 = n1 > 0 ? s.cs + (n1 - 1) * s.step + 1 : s.cs, b1 = min(s.ce, s.cs + n1 * s.step);
+#pragma unroll 1
+  while (a0 < b0 || a1 < b1) {
+    const int32_t m0 = (a0 + b0) >> 1, m1 = (a1 + b1) >> 1;
+    const bool go0 = a0 < b0, go1 = a1 < b1;
+    const uint32_t v0 = go0 ? __ldg(J.fkey + m0) : 0u, v1 = go1 ? __ldg(J.fkey + m1) : 0u;
+    if (go0) {
+      if (v0 < k0)
+        a0 = m0 + 1;
+      else
+        b0 = m0;
+    }
+    if (go1) {
+      if (v1 < k1)
+        a1 = m1 + 1;
+      else
+        b1 = m1;
+    }
+  }
+  *p0 = a0;
+  *p1 = a1;
 }
 
 // Radius of a cell's first shell: R0, scaled down in dense cells by the local density,
@@ -242,20 +285,18 @@ __device__ __forceinline__ double first_radius(const Job& J, D3 x, int lane) {
   uint32_t q[3] = {0u, 0u, 0u};
   for (int i = 0; i < dim; i++) q[i] = fine_q(xa[i], J.ga[i], J.ginv[i], c[i], B);
   const uint32_t key = morton(dim, q[0], q[1], q[2]);
-  int cl = 0;
-  if (lane <= B) {
-    const int sh = dim * (B - lane);
-    const uint32_t klo = (key >> sh) << sh;
-    const int32_t a = fkey_lower_bound(J, cs, ce, klo);
-    cl = fkey_lower_bound(J, a, ce, klo + (1u << sh)) - a;
-  }
+  const int sh = dim * (B - min(lane, B));
+  const uint32_t klo = (key >> sh) << sh;
+  int32_t pa, pb;
+  dense_bounds(J, dense_search(J, cs, ce, lane), klo, klo + (1u << sh), &pa, &pb);
+  const int cl = pb - pa;
   const unsigned bal = __ballot_sync(FULL, lane <= B && cl >= 8);
   if (bal == 0u) return J.R0;
   const int L = 31 - __clz(bal);
   const int cnt = __shfl_sync(FULL, cl, L);
-  const double ratio = (double)cnt * exp2((double)(dim * L)) / J.ppc_mean;
-  if (!(ratio > 1.0)) return J.R0;
-  return J.R0 * pow(ratio, -1.0 / dim);
+  const float ratio = (float)cnt * (float)(1u << (dim * L)) / (float)J.ppc_mean;
+  if (!(ratio > 1.0f)) return J.R0;
+  return J.R0 * (double)exp2f(log2f(ratio) * (-1.0f / dim));
 }
 
 template <int CMAX>
@@ -413,6 +454,78 @@ __device__ __forceinline__ int job_of(const JobTable& T, int pos) {
   return a;
 }
 
+// The elements of the segments [0, nsegs) of B (spref: running element counts) that lie in
+// the shell, appended to its `count` entries; beyond: this lane saw one past its radius.
+struct ShellCount {
+  int count, beyond;
+};
+template <int CMAX, bool BIG, bool DENSE, bool CODE_ONLY>
+__device__ __forceinline__ ShellCount flush_segments(const Job& J, ShellBuf<CMAX>& B, int lane, D3 x, double R2,
+                                                     double lo2, int nsegs, int total, int count, int stop,
+                                                     char* big) {
+  int beyond = 0;
+  auto pass = [&](int t0) {
+    const int t = t0 + lane;
+    bool keep = false;
+    double d2 = 0.0;
+    uint32_t tie = 0;
+    int s = 0;
+    if (t < total) {
+      int a = 0, b = nsegs - 1;
+      while (a < b) {
+        int mid = (a + b + 1) >> 1;
+        if (B.spref[mid] <= t)
+          a = mid;
+        else
+          b = mid - 1;
+      }
+      s = B.sstart[a] + (t - B.spref[a]);
+      const int code = B.scode[a];
+      const double px = __ldg(J.sx + s), py = __ldg(J.sy + s), pz = __ldg(J.sz + s);
+      const int orig = CODE_ONLY ? 0 : __ldg(J.sid + s);
+      if (J.periodic) {
+        const double ddx = (x.x + J.qshift[code][0]) - px;
+        const double ddy = (x.y + J.qshift[code][1]) - py;
+        const double ddz = (x.z + J.qshift[code][2]) - pz;
+        d2 = ddx * ddx + ddy * ddy + ddz * ddz;
+      } else {
+        D3 dd = sub(D3{px, py, pz}, x);
+        d2 = dot(dd, dd);
+      }
+      keep = (d2 >= lo2) && (d2 < R2);
+      beyond |= (d2 >= R2);
+      tie = CODE_ONLY ? (uint32_t)code : (uint32_t)orig * 27u + (uint32_t)code;
+    }
+    const unsigned bal = __ballot_sync(FULL, keep);
+    const int pos = count + __popc(bal & lanemask_lt());
+    if (keep && pos < CMAX) {
+      B.key[pos] = (unsigned long long)__double_as_longlong(d2);
+      B.tie[pos] = tie;
+      B.cpos[pos] = s;
+    } else if (BIG && keep && big != nullptr && pos < BIG_CAP) {
+      const BigView V = big_view(big);
+      V.keyA[pos] = (unsigned long long)__double_as_longlong(d2);
+      V.tieA[pos] = tie;
+      V.cposA[pos] = s;
+    }
+    count += __popc(bal);
+  };
+  if (DENSE) {
+#pragma unroll 1
+    for (int t0 = 0; t0 < total && count <= stop; t0 += 32) pass(t0);
+  } else {
+    for (int t0 = 0; t0 < total && count <= stop; t0 += 32) pass(t0);
+  }
+  __syncwarp();
+  return {count, beyond};
+}
+// one copy where a gather reaches it from several places (see gather_shell_impl)
+template <int CMAX, bool BIG, bool CODE_ONLY>
+__device__ __noinline__ ShellCount flush_call(const Job& J, ShellBuf<CMAX>& B, int lane, D3 x, double R2,
+                                              double lo2, int nsegs, int total, int count, int stop, char* big) {
+  return flush_segments<CMAX, BIG, true, CODE_ONLY>(J, B, lane, x, R2, lo2, nsegs, total, count, stop, big);
+}
+
 // Gathers every stream element (generator, periodic image) with lo2 <= d2 < R*R into
 // B (unsorted) and returns how many there are (may exceed CMAX; once the count passes
 // stop the gather ends early and returns a count above stop).  With BIG and a slot,
@@ -424,9 +537,14 @@ __device__ __forceinline__ int job_of(const JobTable& T, int pos) {
 //
 // Grid rows (y, z) go to lanes; a lane turns the cells of its row that the ball
 // reaches into contiguous segments of sorted positions (one per periodic image).  A
-// segment that contains a dense cell (J.dprefix) is deferred: its cells are then
-// visited one by one, and a dense cell contributes the octree cells that the shell
+// segment that contains a dense cell (J.dprefix) is deferred: its runs of sparse cells
+// are then taken a run per lane and its dense cells one by one, and a dense cell contributes the octree cells that the shell
 // reaches.  Without the ball test (all images enumerated) every cell counts whole.
+// What bounds the two-level form is instruction fetch (more than half of a warp's stalls):
+// its code is kept small, with rolled loops and one called copy of flush_segments, where
+// the one-level form, a third of the size, is faster unrolled (128^3 Poisson shells 7.6 ms,
+// rolled 8.2).  8.4 M generators, half of them in clumps: 843 -> 780 ms for the build, with
+// dense_search and the sparse runs of a deferred segment taken together.
 template <int CMAX, bool BIG, bool DENSE, bool CODE_ONLY>
 __device__ __noinline__ int gather_shell_impl(const Job& J, ShellBuf<CMAX>& B, int lane, D3 x, double R,
                                               double lo2, const double* ext, bool* exhausted,
@@ -481,54 +599,11 @@ __device__ __noinline__ int gather_shell_impl(const Job& J, ShellBuf<CMAX>& B, i
   };
 
   // the elements of the segments [0, nsegs) of B (spref: running element counts)
-  auto flush = [&](int nsegs_total, int total) {
-    for (int t0 = 0; t0 < total && count <= stop; t0 += 32) {
-      const int t = t0 + lane;
-      bool keep = false;
-      double d2 = 0.0;
-      uint32_t tie = 0;
-      int s = 0;
-      if (t < total) {
-        int a = 0, b = nsegs_total - 1;
-        while (a < b) {
-          int mid = (a + b + 1) >> 1;
-          if (B.spref[mid] <= t)
-            a = mid;
-          else
-            b = mid - 1;
-        }
-        s = B.sstart[a] + (t - B.spref[a]);
-        const int code = B.scode[a];
-        const double px = __ldg(J.sx + s), py = __ldg(J.sy + s), pz = __ldg(J.sz + s);
-        const int orig = CODE_ONLY ? 0 : __ldg(J.sid + s);
-        if (J.periodic) {
-          const double ddx = (x.x + J.qshift[code][0]) - px;
-          const double ddy = (x.y + J.qshift[code][1]) - py;
-          const double ddz = (x.z + J.qshift[code][2]) - pz;
-          d2 = ddx * ddx + ddy * ddy + ddz * ddz;
-        } else {
-          D3 dd = sub(D3{px, py, pz}, x);
-          d2 = dot(dd, dd);
-        }
-        keep = (d2 >= lo2) && (d2 < R2);
-        beyond += (d2 >= R2);
-        tie = CODE_ONLY ? (uint32_t)code : (uint32_t)orig * 27u + (uint32_t)code;
-      }
-      const unsigned bal = __ballot_sync(FULL, keep);
-      const int pos = count + __popc(bal & lanemask_lt());
-      if (keep && pos < CMAX) {
-        B.key[pos] = (unsigned long long)__double_as_longlong(d2);
-        B.tie[pos] = tie;
-        B.cpos[pos] = s;
-      } else if (BIG && keep && big != nullptr && pos < BIG_CAP) {
-        const BigView V = big_view(big);
-        V.keyA[pos] = (unsigned long long)__double_as_longlong(d2);
-        V.tieA[pos] = tie;
-        V.cposA[pos] = s;
-      }
-      count += __popc(bal);
-    }
-    __syncwarp();
+  auto flush = [&](int nsegs, int total) {
+    const ShellCount c = DENSE ? flush_call<CMAX, BIG, CODE_ONLY>(J, B, lane, x, R2, lo2, nsegs, total, count, stop, big)
+                               : flush_segments<CMAX, BIG, false, CODE_ONLY>(J, B, lane, x, R2, lo2, nsegs, total, count, stop, big);
+    count = c.count;
+    beyond |= c.beyond;
   };
   // segments of one per lane (len 0: none) into B, then their elements
   auto emit1 = [&](int32_t st0, int32_t len, int code) {
@@ -541,6 +616,16 @@ __device__ __noinline__ int gather_shell_impl(const Job& J, ShellBuf<CMAX>& B, i
     __syncwarp();
     if (bal) flush(__popc(bal), tot);
   };
+  // the level of a dense cell's octree cells: at least half as wide as the shell is thick
+  // (R / 8 at the thinnest), so that a thin shell's octree cells inside the inner radius
+  // drop out
+  int level = 0;
+  if (DENSE) {
+    double hmin = J.gh[0];
+    for (int i = 1; i < J.dim; i++) hmin = fmin(hmin, J.gh[i]);
+    const double r = 2.0 * hmin / (lo2 > 0.0 ? fmax(R - sqrt(lo2), 0.125 * R) : R);
+    level = r >= 2.0 ? min(J.fbits, ilogb(r)) : 0;
+  }
   // the octree cells of dense cell (cx, cy, cz), image (mx, my, mz), that the shell
   // [lo, R) reaches, at the level whose cells are at least half the shell's thickness
   // wide (at most five per axis for a first shell, 33 for the thinnest); a cell that
@@ -548,18 +633,8 @@ __device__ __noinline__ int gather_shell_impl(const Job& J, ShellBuf<CMAX>& B, i
   auto dense_cell = [&](int cx, int cy, int cz, int mx, int my, int mz, int code) {
     const int64_t cc = (int64_t)cx + (int64_t)J.G[0] * (cy + (int64_t)J.G[1] * cz);
     const int32_t cs = __ldg(J.cell_start + cc), ce = __ldg(J.cell_start + cc + 1);
-    if (all) {
-      emit1(cs, lane == 0 ? ce - cs : 0, code);
-      return;
-    }
     const int B = J.fbits, dim = J.dim;
-    double hmin = J.gh[0];
-    for (int i = 1; i < dim; i++) hmin = fmin(hmin, J.gh[i]);
-    // the level: cells at least half as wide as the shell is thick (R / 8 at the
-    // thinnest), so that a thin shell's octree cells inside the inner radius drop out
-    const double span = fmax(R - sqrt(lo2), 0.125 * R);
-    const double r = 2.0 * hmin / span;
-    const int L = r >= 2.0 ? min(B, ilogb(r)) : 0;
+    const int L = all ? 0 : level;
     const int nL = 1 << L;
     const int c3[3] = {cx, cy, cz}, m3[3] = {mx, my, mz};
     int ja[3], jn[3];
@@ -569,11 +644,13 @@ __device__ __noinline__ int gather_shell_impl(const Job& J, ShellBuf<CMAX>& B, i
       clo[i] = cell_lo(i, c3[i], m3[i]);
       chi[i] = cell_hi(i, c3[i], m3[i]);
       base[i] = J.ga[i] + c3[i] * J.gh[i] + m3[i] * J.gw[i];
-      w[i] = J.gh[i] / nL;
+      w[i] = J.gh[i] * (1.0 / nL);  // exact: nL is a power of two
       ja[i] = 0, jn[i] = 1;
       if (i < dim) {
-        const double fa = floor((xa[i] - R - base[i] - J.geps[i]) / w[i]);
-        const double fb = floor((xa[i] + R - base[i] + J.geps[i]) / w[i]);
+        // (a millionth of a cell wider than needed, against the rounding of ginv)
+        const double iw = J.ginv[i] * nL;
+        const double fa = floor((xa[i] - R - base[i] - J.geps[i]) * iw - 1e-6);
+        const double fb = floor((xa[i] + R - base[i] + J.geps[i]) * iw + 1e-6);
         const int lo_j = fa < 0.0 ? 0 : (fa > nL - 1 ? nL - 1 : (int)fa);
         const int hi_j = fb > nL - 1 ? nL - 1 : (fb < 0.0 ? 0 : (int)fb);
         ja[i] = lo_j, jn[i] = hi_j - lo_j + 1;
@@ -582,11 +659,15 @@ __device__ __noinline__ int gather_shell_impl(const Job& J, ShellBuf<CMAX>& B, i
     const int sh = dim * (B - L);
     const int ncl = jn[0] * jn[1] * jn[2];
     const double lo2p = lo2 * (1.0 - 1e-9);
+    const DenseSearch ds = dense_search(J, cs, ce, lane);
+#pragma unroll 1
     for (int r0 = 0; r0 < ncl && count <= stop; r0 += 32) {
       const int t = r0 + lane;
-      int32_t st0 = 0, len = 0;
+      bool in = false;
+      uint32_t klo = 0u;
       if (t < ncl) {
-        const int j[3] = {ja[0] + t % jn[0], ja[1] + (t / jn[0]) % jn[1], ja[2] + t / (jn[0] * jn[1])};
+        const unsigned t1 = (unsigned)t / (unsigned)jn[0], t2 = t1 / (unsigned)jn[1];
+        const int j[3] = {ja[0] + t - (int)t1 * jn[0], ja[1] + (int)(t1 - t2 * jn[1]), ja[2] + (int)t2};
         double dmin2 = 0.0, dmax2 = 0.0;
 #pragma unroll
         for (int i = 0; i < 3; i++) {
@@ -600,13 +681,12 @@ __device__ __noinline__ int gather_shell_impl(const Job& J, ShellBuf<CMAX>& B, i
           dmin2 += dn * dn;
           dmax2 += df * df;
         }
-        if (dmin2 < R2v && !(dmax2 < lo2p)) {
-          const uint32_t klo = morton(dim, (uint32_t)j[0], (uint32_t)j[1], (uint32_t)j[2]) << sh;
-          st0 = fkey_lower_bound(J, cs, ce, klo);
-          len = fkey_lower_bound(J, st0, ce, klo + (1u << sh)) - st0;
-        }
+        in = all || (dmin2 < R2v && !(dmax2 < lo2p));
+        if (in) klo = morton(dim, (uint32_t)j[0], (uint32_t)j[1], (uint32_t)j[2]) << sh;
       }
-      emit1(st0, len, code);
+      int32_t st0, st1;
+      dense_bounds(J, ds, klo, in ? klo + (1u << sh) : 0u, &st0, &st1);
+      emit1(st0, st1 - st0, code);
     }
   };
 
@@ -704,10 +784,32 @@ __device__ __noinline__ int gather_shell_impl(const Job& J, ShellBuf<CMAX>& B, i
     }
     __syncwarp();
     flush(nsegs_total, total);
-    // the deferred ranges, cell by cell (a sparse cell is one segment)
+    // the deferred ranges: their runs of sparse cells, a run per lane at a time, then
+    // their dense cells one by one
+#pragma unroll 1
     for (int im = 0; im < (DENSE ? 3 : 0); im++) {
       unsigned pend = __ballot_sync(FULL, dfr[im] >= 0);
-      while (pend) {
+      if (pend == 0u) continue;
+      {
+        int c = dfr[im] >= 0 ? dfr[im] & 0xffff : 1;
+        const int c1 = dfr[im] >= 0 ? dfr[im] >> 16 : 0;
+        const int64_t rowbase = (int64_t)J.G[0] * (cy + (int64_t)J.G[1] * cz);
+        const int code = im + 3 * (my + 1) + 9 * (mz + 1);
+        do {
+#pragma unroll 1
+          while (c <= c1 && __ldg(J.cell_dense + rowbase + c)) c++;
+          int32_t st0 = 0, len = 0;
+          if (c <= c1) {
+            st0 = __ldg(J.cell_start + rowbase + c);
+#pragma unroll 1
+            while (c <= c1 && !__ldg(J.cell_dense + rowbase + c)) c++;
+            len = __ldg(J.cell_start + rowbase + c) - st0;
+          }
+          __syncwarp();
+          emit1(st0, len, code);
+        } while (__any_sync(FULL, c <= c1) && count <= stop);
+      }
+      while (pend && count <= stop) {
         const int src = __ffs(pend) - 1;
         pend &= pend - 1;
         const int rg = __shfl_sync(FULL, dfr[im], src);
@@ -716,14 +818,10 @@ __device__ __noinline__ int gather_shell_impl(const Job& J, ShellBuf<CMAX>& B, i
         const int mx = im - 1;
         const int code = (mx + 1) + 3 * (rmy + 1) + 9 * (rmz + 1);
         const int64_t rowbase = (int64_t)J.G[0] * (ry + (int64_t)J.G[1] * rz);
-        for (int c = rg & 0xffff; c <= (rg >> 16) && count <= stop; c++) {
-          if (__ldg(J.cell_dense + rowbase + c)) {
-            dense_cell(c, ry, rz, mx, rmy, rmz, code);
-          } else {
-            const int32_t ps = __ldg(J.cell_start + rowbase + c);
-            const int32_t pe = __ldg(J.cell_start + rowbase + c + 1);
-            emit1(ps, lane == 0 ? pe - ps : 0, code);
-          }
+        for (int c0 = rg & 0xffff; c0 <= (rg >> 16); c0 += 32) {
+          unsigned dense = __ballot_sync(FULL, c0 + lane <= (rg >> 16) && __ldg(J.cell_dense + rowbase + c0 + lane));
+          for (; dense && count <= stop; dense &= dense - 1)
+            dense_cell(c0 + __ffs(dense) - 1, ry, rz, mx, rmy, rmz, code);
         }
       }
     }

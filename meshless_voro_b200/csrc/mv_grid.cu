@@ -535,6 +535,16 @@ __global__ void batch_local_starts_kernel(int32_t* __restrict__ start, int64_t n
   start[c] -= pos[batch_find(cbase, nj, c)];
 }
 
+// a tessellation without dense cells takes the one-level search, as it would by itself
+__global__ void batch_levels_kernel(Job* __restrict__ jobs, const int32_t* __restrict__ dprefix,
+                                    const int32_t* __restrict__ cbase, int nj) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= nj || dprefix[cbase[j + 1]] != dprefix[cbase[j]]) return;
+  jobs[j].dprefix = nullptr;
+  jobs[j].cell_dense = nullptr;
+  jobs[j].fkey = nullptr;
+}
+
 // first face and first connection of each tessellation (j = nj: the totals)
 __global__ void batch_bases_kernel(const int64_t* __restrict__ face_off, const int64_t* __restrict__ conn_off,
                                    const int32_t* __restrict__ pos, int nj, int64_t* __restrict__ fbase,
@@ -632,8 +642,8 @@ void launch_grid(const double* gen, int n, const int G[3], const double a[3], co
 // cells (flags and their running count).  The host reads the number of dense cells,
 // then calls launch_grid_dense (or scatters coarse-only).  Returns the launches.
 int launch_grid_coarse(const double* gen, int n, const int G[3], const double a[3],
-                        const double inv[3], int32_t* cid, int32_t* count, int32_t* start,
-                        int32_t* dflag, int32_t* dprefix, int dim, long long* scan_tmp, cudaStream_t st) {
+                       const double inv[3], int32_t* cid, int32_t* count, int32_t* start,
+                       int32_t* dflag, int32_t* dprefix, int dim, long long* scan_tmp, cudaStream_t st) {
   GridParams gp;
   for (int i = 0; i < 3; i++) gp.G[i] = G[i], gp.a[i] = a[i], gp.inv[i] = inv[i];
   gp.dim = dim;
@@ -737,6 +747,10 @@ cudaError_t launch_batch_sort(const double* gen, int n, const int32_t* pos, cons
   }
   batch_local_starts_kernel<<<nblk(ncell, 256), 256, 0, st>>>(start, ncell, cbase, pos, nj);
   return cudaGetLastError();
+}
+
+void launch_batch_levels(Job* jobs, const int32_t* dprefix, const int32_t* cbase, int nj, cudaStream_t st) {
+  batch_levels_kernel<<<nblk(nj, 256), 256, 0, st>>>(jobs, dprefix, cbase, nj);
 }
 
 void launch_batch_localize(FaceArrays& f, int64_t F, const int64_t* face_off, int64_t* conn_off,
