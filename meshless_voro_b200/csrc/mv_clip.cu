@@ -1070,6 +1070,9 @@ int clip_blocks_per_sm(int precision, bool wide) {
   return wide ? clip_occupancy<ClipWide>(precision) : clip_occupancy<ClipFirst>(precision);
 }
 
+// Cells a block of the wide tier works on at a time.
+int clip_cells_per_block() { return ClipWide::WARPS * ClipWide::NG; }
+
 template <class T>
 static cudaError_t launch_clip_t(const Job& J, StageJob SJ, const JobTable& TB, int resident, cudaStream_t st) {
   // four cells per warp once the resident grid is full; a smaller build leaves groups idle

@@ -209,12 +209,14 @@ __global__ void __launch_bounds__(32 * WARPS, MV_SHELL_MINB)
 // The wide round: cells the first round could not close get a shell of up to WIDE_CMAX
 // candidates (about eight times the first one), sorted in shared memory.  Cells the
 // wide round cannot close either go to the fused kernel.
-// Its radius is found by count.  In a build without dense cells a cell that the first shell
-// did not close has a shallow void beside it: 1.4 radii, about 250 candidates, close all but
-// the few whose cell outgrows the tier, and sort in a quarter of the time (s. 16,736 cells of
-// 128^3 Poisson generators: 1.07 -> 0.40 ms, 54 cells of 4,096: 0.10 -> 0.06 ms).  Beside
-// clumps a cell may need thousands, and what a larger shell closes here costs less than in
-// the fused kernel (8.4 M clustered generators: 843 ms, with the small shells 853).
+// Its radius is found by count.  In a periodic build without dense cells a cell that the
+// first shell did not close has a shallow void beside it: 1.4 radii, about 250 candidates,
+// close all but the few whose cell outgrows the tier, and sort in a quarter of the time
+// (16,736 cells of 128^3 Poisson generators: 1.07 -> 0.40 ms, 54 cells of 4,096: 0.10 ->
+// 0.06 ms).  At a wall half of a shell is empty (6,000 generators in a box: two cells stay
+// open with it, and cost 0.17 ms in the fused kernel), and beside clumps a cell may need
+// thousands: there a shell of two radii, about 740 candidates, closes more than it costs
+// (8.4 M clustered generators: 843 ms, with the small shells 853).
 constexpr int WIDE_CMAX = 1024;
 constexpr int WIDE_WARPS = 4;
 constexpr size_t WIDE_SMEM = sizeof(ShellBuf<WIDE_CMAX>) * WIDE_WARPS;
@@ -282,10 +284,10 @@ __global__ void __launch_bounds__(32 * WARPS, 3)
     }
     const D3 x = load_gen(J, self);
     bool all = false;
-    const bool clumps = J.fkey != nullptr;
-    const int least = clumps ? 384 : 128;          // widened below this many candidates
-    const double aim = clumps ? 768.0 : 256.0;
-    double R = (clumps ? 2.0 : 1.4) * first_radius(J, x, lane);
+    const bool even = J.fkey == nullptr && J.periodic;
+    const int least = even ? 128 : 384;  // widened below this many candidates
+    const double aim = even ? 256.0 : 768.0;
+    double R = (even ? 1.4 : 2.0) * first_radius(J, x, lane);
     int cnt = gather_shell<WIDE_CMAX>(J, B, lane, x, R, 0.0, ext, &all, 4 * WIDE_CMAX);
     for (int it = 0; it < 6; it++) {
       double f;

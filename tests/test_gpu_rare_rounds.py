@@ -52,3 +52,21 @@ def test_many_faced_cells(gpu_ctx, oracle, stars, precision):
     g = np.concatenate([g, c, (c[:, None] + 0.14 * v).reshape(-1, 3)])
     st = _check(gpu_ctx, oracle, rng.permutation(g), 3, False, precision)
     assert st is None or st["overflow_cells"] >= stars
+
+
+@pytest.mark.parametrize("precision", ["filtered", "fp64"])
+@pytest.mark.parametrize("n", [800, 7103, 7104, 7105, 9000, 24_000])
+@pytest.mark.parametrize("periodic", [False, True])
+def test_tier_of_the_first_round(gpu_ctx, oracle, n, periodic, precision):
+    """Around the size up to which the first round takes the wide tier: Poisson cells, and a
+    cell of some 40 faces, which only the wide tier holds."""
+    rng = np.random.default_rng(n)
+    v = rng.normal(size=(44, 3))
+    v /= np.linalg.norm(v, axis=1)[:, None]
+    c = np.array([0.4, 0.5, 0.6])
+    r = 1.6 * n ** (-1.0 / 3.0)
+    g = rng.random((2 * n, 3))
+    g = g[np.sqrt(((g - c) ** 2).sum(axis=1)) > 1.15 * r][: n - 45]
+    g = rng.permutation(np.concatenate([g, [c], c + r * (1.0 + 0.03 * rng.random((44, 1))) * v]))
+    assert len(g) == n
+    _check(gpu_ctx, oracle, g, 3, periodic, precision)
