@@ -60,12 +60,16 @@ struct ClipTier {
   static constexpr int WIN = 2 * G_;    // candidates in the window (refilled G at a time)
   static constexpr int RMAX = 32;       // removed vertices, ring edges
   static constexpr int NC = VMAX_ / G_; // vertices per lane
+  // bytes per plane: words, and the successor of a node outside the ring.  No plane has the
+  // number PMAX, so its byte is free: it stays NONE, and a walk that leaves a broken ring
+  // goes on inside the table
+  static constexpr int PW = (PMAX_ + 4) / 4;
+  static constexpr unsigned NONE = PMAX_;
+  static constexpr uint32_t NONE4 = 0x01010101u * NONE;
   static_assert(G_ == 8 && VMAX_ % (2 * G_) == 0 && VMAX_ <= 64 && PMAX_ < 255, "tier");
 };
 using ClipFirst = ClipTier<MV_CLIP_G, MV_CLIP_VMAX, MV_CLIP_PMAX, MV_CLIP_WARPS, MV_CLIP_MINB>;
 using ClipWide = ClipTier<MV_CLIP_G, 64, 64, MV_CLIP_WARPS, 6>;
-
-constexpr unsigned RING_NONE = 0xffu;  // successor of a node outside the ring
 
 __device__ __forceinline__ uint32_t pack_dual(int i, int j, int k) {
   return (uint32_t)i | ((uint32_t)j << 8) | ((uint32_t)k << 16);
@@ -86,8 +90,8 @@ struct GroupPlanes {
   float2 wc[T::WIN];   // window: f32 bound of the filter without its A term, |x - ngb| rounded up
   uint32_t rd[T::RMAX];  // duals of the removed vertices, in the reference's order
   // byte per plane: the removed triangles that hold it (zero between uses), and its
-  // successor (RING_NONE between uses) and predecessor on the ring
-  uint32_t plm[(T::PMAX + 4) / 4], ring[(T::PMAX + 4) / 4], back[(T::PMAX + 4) / 4];
+  // successor (NONE between uses) and predecessor on the ring
+  uint32_t plm[T::PW], ring[T::PW], back[T::PW];
   uint16_t pidx[T::PMAX + 1];  // candidate of each bisector plane
   __device__ __forceinline__ D3 normal(int k) const { return {pxy[k].x, pxy[k].y, pzd[k].x}; }
   __device__ __forceinline__ double d(int k) const { return pzd[k].y; }
@@ -455,7 +459,7 @@ __device__ __noinline__ unsigned ring_wide(SM& S, int gl, int gbase, bool on, in
   uint8_t* const rptr = reinterpret_cast<uint8_t*>(S.ring);
   if (on)
 #pragma unroll 1
-    for (int i = gl; i < (T::PMAX + 4) / 4; i += G) S.ring[i] = ~0u;
+    for (int i = gl; i < T::PW; i += G) S.ring[i] = T::NONE4;
   __syncwarp();
   const uint32_t d0 = on ? S.rd[0] : 0u;
   int start = d0 & 0xff, E = 3;
@@ -475,7 +479,7 @@ __device__ __noinline__ unsigned ring_wide(SM& S, int gl, int gbase, bool on, in
       const unsigned t0 = du & 0xff, t1 = (du >> 8) & 0xff, t2 = (du >> 16) & 0xff;
       const unsigned p0 = rptr[t0], p1 = rptr[t1], p2 = rptr[t2];
       const bool s0 = p2 == t1, s1 = p0 == t2, s2 = p1 == t0;
-      const bool o0 = p0 == RING_NONE, o1 = p1 == RING_NONE, o2 = p2 == RING_NONE;
+      const bool o0 = p0 == T::NONE, o1 = p1 == T::NONE, o2 = p2 == T::NONE;
       const bool x0 = s0 && (o0 || s2), x1 = s1 && (o1 || s0), x2 = s2 && (o2 || s1);
       const bool can = du != 0u && (x0 || x1 || x2);
       const bool grow_l = x0 ? o0 : (x1 ? o1 : o2);
@@ -488,7 +492,7 @@ __device__ __noinline__ unsigned ring_wide(SM& S, int gl, int gbase, bool on, in
       const bool grow = (win >> 24) != 0u, did = step && bal != 0u;
       if (did && gl == 0) {
         rptr[tc] = (uint8_t)ta;
-        rptr[grow ? ta : tb] = (uint8_t)(grow ? tb : RING_NONE);
+        rptr[grow ? ta : tb] = (uint8_t)(grow ? tb : T::NONE);
         S.rd[base + src] = head;  // swap(i, found): position i is done with
       }
       if (did) E += grow ? 1 : -1;
@@ -510,7 +514,7 @@ __device__ __noinline__ unsigned ring_wide(SM& S, int gl, int gbase, bool on, in
     }
     __syncwarp(GM << gbase);
 #pragma unroll 1
-    for (int i = gl; i < (T::PMAX + 4) / 4; i += G) S.ring[i] = ~0u;
+    for (int i = gl; i < T::PW; i += G) S.ring[i] = T::NONE4;
   }
   __syncwarp();
   return ok ? (unsigned)E | (moved ? 1u << 16 : 0u) : 0u;
@@ -685,7 +689,7 @@ __global__ void __launch_bounds__(32 * T::WARPS, T::MINB)
         S.pzd[i] = make_double2(J.bn[i][2], J.bd[i]);
       }
 #pragma unroll 1
-      for (int i = gl; i < (T::PMAX + 4) / 4; i += G) S.plm[i] = 0u, S.ring[i] = ~0u, S.back[i] = 0u;
+      for (int i = gl; i < T::PW; i += G) S.plm[i] = 0u, S.ring[i] = T::NONE4, S.back[i] = 0u;
 #pragma unroll 1
       for (int q = gl; q < T::VMAX; q += G) S.set_none(q, x);
     }
@@ -915,7 +919,7 @@ __global__ void __launch_bounds__(32 * T::WARPS, T::MINB)
         // the ring starts at the first triangle's first node; when that becomes interior, at
         // the node before it in the triangle that closed its fan, which takes the reference's
         // order to tell
-        moved = hit && !wide && next[start] == RING_NONE;
+        moved = hit && !wide && next[start] == T::NONE;
         if (__any_sync(FULL, moved)) {
           if (!moved) N = 0u;
           start = ring_start(du, M, N, gl, gbase, start);
@@ -935,9 +939,9 @@ __global__ void __launch_bounds__(32 * T::WARPS, T::MINB)
         // one cycle through the start: each node's successor is the next lane's node
         const int un = __shfl_sync(FULL, u, gl + 1 < E ? gl + 1 : 0, G);
         const bool on = hit && !wide && gl < E;
-        const bool bad = on && (w != un || u >= (int)RING_NONE || (gl > 0 && u == start));
+        const bool bad = on && (w != un || u == (int)T::NONE || (gl > 0 && u == start));
         __syncwarp();
-        if (on) next[u] = (uint8_t)RING_NONE;
+        if (on) next[u] = (uint8_t)T::NONE;
         const unsigned broken = __ballot_sync(FULL, bad) & gmask;
         wide = wide || broken != 0u;
       }
