@@ -914,7 +914,9 @@ __global__ void __launch_bounds__(32 * T::WARPS, T::MINB)
         if (b2) next[t0] = (uint8_t)t1, prev[t1] = (uint8_t)t0;
         if (mine) pb[t0] = 0, pb[t1] = 0, pb[t2] = 0;
         E = __popc(gballot(b0)) + __popc(gballot(b1)) + __popc(gballot(b2));
-        wide = hit && (r > G || E > G);
+        // a cut that removes every vertex leaves no edge: what the reference's loop makes of
+        // it (a ring of two nodes) only that loop tells
+        wide = hit && (r > G || E > G || E < 3);
         __syncwarp();
         // the ring starts at the first triangle's first node; when that becomes interior, at
         // the node before it in the triangle that closed its fan, which takes the reference's
@@ -946,8 +948,8 @@ __global__ void __launch_bounds__(32 * T::WARPS, T::MINB)
         wide = wide || broken != 0u;
       }
       if (__any_sync(FULL, wide)) {
-        // more removed vertices or ring edges than lanes (or an order that only the reference's
-        // own loop decides): the ring through shared memory
+        // more removed vertices or ring edges than lanes, or a ring that only the reference's
+        // own loop decides: the ring through shared memory
         const unsigned got = ring_wide<T>(S, gl, gbase, wide && hit, r);
         if (wide) E = got & 0xffff, moved = got >> 16;
         if (wide && hit && got == 0u) {
