@@ -224,6 +224,10 @@ __device__ __forceinline__ double group_max(double m) {
   return m;
 }
 
+// Squared radii from here on are within f32 rounding of their f64 values (below, the
+// squares of the coordinates lose bits or vanish: cells smaller than 1e-15).
+constexpr float SQUARE_MIN = 1e-30f;
+
 // The safety radius (convex_cell.rs:443-453) of a group's nv vertices in f64, given their
 // largest squared radius in f32: only the vertices within f32 rounding of it can be the
 // farthest.
@@ -232,7 +236,7 @@ __device__ __noinline__ double exact_radius(const SM& S, int gl, int nv, float m
   double m = 0.0;
 #pragma unroll 1
   for (int q = gl; q < nv; q += G) {
-    if (S.radius2_f32(q, x, dim) < m2 * 0.999998f) continue;
+    if (m2 >= SQUARE_MIN && S.radius2_f32(q, x, dim) < m2 * 0.999998f) continue;
     const double r2 = radius2(S.loc(q), x, dim);
     m = r2 > m ? r2 : m;
   }
@@ -617,9 +621,11 @@ __global__ void __launch_bounds__(32 * T::WARPS, T::MINB)
     float su;  // within 1e-6 of 2 sqrt(m)
     asm("sqrt.approx.f32 %0, %1;" : "=f"(su) : "f"(m));
     su += su;
-    // out of the range where su is accurate, every candidate is compared in f64
-    su_lo = m >= 1e-30f && m <= 1e37f ? su * 0.999998f : 0.f;
-    su_hi = su * 1.000002f;
+    // out of the range where su is accurate (a square near the smallest f32 or the largest),
+    // every candidate is compared in f64
+    const bool fine = m >= SQUARE_MIN && m <= 1e37f;
+    su_lo = fine ? su * 0.999998f : 0.f;
+    su_hi = fine ? su * 1.000002f : INFINITY;
     // |v - x| <= A32 (the extruded dimensions add up to 0.5 each)
     A32 = 0.5000001f * su_hi + (dim == 3 ? 0.f : (dim == 2 ? 0.51f : 0.7212f));
     if (!(A32 <= 1e15f)) A32 = INFINITY;
