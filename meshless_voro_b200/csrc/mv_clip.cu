@@ -233,10 +233,11 @@ constexpr float SQUARE_MIN = 1e-30f;
 // farthest.
 template <int G, class SM>
 __device__ __noinline__ double exact_radius(const SM& S, int gl, int nv, float m2, D3 x, int dim) {
+  const float least = m2 >= SQUARE_MIN ? m2 * 0.999998f : 0.f;
   double m = 0.0;
 #pragma unroll 1
   for (int q = gl; q < nv; q += G) {
-    if (m2 >= SQUARE_MIN && S.radius2_f32(q, x, dim) < m2 * 0.999998f) continue;
+    if (S.radius2_f32(q, x, dim) < least) continue;
     const double r2 = radius2(S.loc(q), x, dim);
     m = r2 > m ? r2 : m;
   }
@@ -621,11 +622,11 @@ __global__ void __launch_bounds__(32 * T::WARPS, T::MINB)
     float su;  // within 1e-6 of 2 sqrt(m)
     asm("sqrt.approx.f32 %0, %1;" : "=f"(su) : "f"(m));
     su += su;
-    // out of the range where su is accurate (a square near the smallest f32 or the largest),
-    // every candidate is compared in f64
-    const bool fine = m >= SQUARE_MIN && m <= 1e37f;
-    su_lo = fine ? su * 0.999998f : 0.f;
-    su_hi = fine ? su * 1.000002f : INFINITY;
+    // out of the range where su is accurate (a square near the smallest f32 or the largest)
+    // the bounds are no numbers, which tells nothing of any candidate: all are compared in f64
+    if (!(m >= SQUARE_MIN && m <= 1e37f)) su = NAN;
+    su_lo = su * 0.999998f;
+    su_hi = su * 1.000002f;
     // |v - x| <= A32 (the extruded dimensions add up to 0.5 each)
     A32 = 0.5000001f * su_hi + (dim == 3 ? 0.f : (dim == 2 ? 0.51f : 0.7212f));
     if (!(A32 <= 1e15f)) A32 = INFINITY;
@@ -920,9 +921,7 @@ __global__ void __launch_bounds__(32 * T::WARPS, T::MINB)
         if (b2) next[t0] = (uint8_t)t1, prev[t1] = (uint8_t)t0;
         if (mine) pb[t0] = 0, pb[t1] = 0, pb[t2] = 0;
         E = __popc(gballot(b0)) + __popc(gballot(b1)) + __popc(gballot(b2));
-        // a cut that removes every vertex leaves no edge: what the reference's loop makes of
-        // it (a ring of two nodes) only that loop tells
-        wide = hit && (r > G || E > G || E < 3);
+        wide = hit && (r > G || E > G);
         __syncwarp();
         // the ring starts at the first triangle's first node; when that becomes interior, at
         // the node before it in the triangle that closed its fan, which takes the reference's
@@ -931,6 +930,9 @@ __global__ void __launch_bounds__(32 * T::WARPS, T::MINB)
         if (__any_sync(FULL, moved)) {
           if (!moved) N = 0u;
           start = ring_start(du, M, N, gl, gbase, start);
+          // a cut that removes every vertex leaves no edge (and no first node on one): what the
+          // reference's loop makes of it, a ring of two nodes, only that loop tells
+          wide = wide || (moved && E < 3);
         }
       }
       int u, w;
