@@ -55,8 +55,8 @@ cudaError_t launch_append_range(int32_t* dst, int32_t first, int32_t count, cuda
 constexpr int64_t STAGE_PROBE_CELLS = 16384;
 int64_t stage_record_words(int np, int nv);
 // mv_grid.cu
-void launch_prep(const double* xyz, int n, int dim, double* gen, unsigned long long* ext_keys,
-                 double* ext, int* bad, cudaStream_t st);
+void launch_prep(const double* xyz, int n, int dim, const double anchor[3], const double width[3], double* gen,
+                 unsigned long long* ext_keys, double* ext, int32_t* outside, int* bad, cudaStream_t st);
 int launch_grid_coarse(const double* gen, int n, const int G[3], const double a[3],
                        const double inv[3], int32_t* cid, int32_t* count, int32_t* start,
                        int32_t* dflag, int32_t* dprefix, int dim, long long* scan_tmp, cudaStream_t st);
@@ -789,7 +789,7 @@ int build_device_impl(mv_context* ctx, const double* d_xyz, const uint8_t* d_mas
   e |= ensure(ctx, W.cell_start, 4 * (ncell + 1));
   e |= ensure(ctx, W.cell_fill, 4 * (ncell + 1));
   e |= ensure(ctx, W.dflag, 4 * (ncell + 1));
-  e |= ensure(ctx, W.dprefix, 4 * (ncell + 1));
+  e |= ensure(ctx, W.dprefix, 4 * (ncell + 2));
   e |= ensure(ctx, W.scan_tmp, 8 * (scan_tmp_elems(std::max<int64_t>(ncell + 1, N)) + 64));
   e |= ensure(ctx, W.volume, 8 * N);
   e |= ensure(ctx, W.centroid, 24 * N);
@@ -837,12 +837,15 @@ int build_device_impl(mv_context* ctx, const double* d_xyz, const uint8_t* d_mas
     // ---- generators + grid (replaces build_rtree, rtree_nn.rs:6-8) ----
     MV_CUDA(cudaEventRecord(ctx->ev[0], st));
     launches = 3;  // prep, extent, scatter
-    launch_prep(d_xyz, ni, s.dim, P<double>(W.gen), C->ext_keys, C->ext, &C->bad_input, st);
+    // one readback: the number of dense cells, and whether generators lie outside the box
+    int32_t got[2] = {0, 0};
+    launch_prep(d_xyz, ni, s.dim, s.anchor, s.width, P<double>(W.gen), C->ext_keys, C->ext,
+                P<int32_t>(W.dprefix) + ncell + 1, &C->bad_input, st);
     launches += launch_grid_coarse(P<double>(W.gen), ni, s.G, s.anchor, s.ginv, P<int32_t>(W.cid),
                                    P<int32_t>(W.cell_count), P<int32_t>(W.cell_start), P<int32_t>(W.dflag),
                                    P<int32_t>(W.dprefix), s.dim, P<long long>(W.scan_tmp), st);
-    int32_t ndense = 0;
-    MV_RB(&ndense, P<int32_t>(W.dprefix) + ncell, 4);
+    MV_RB(got, P<int32_t>(W.dprefix) + ncell, 8);
+    const int32_t ndense = got[0];
     if (ndense > 0) {
       // clustered input: the dense cells are ordered by Morton key (a radix sort)
       const size_t sort_bytes = grid_dense_sort_bytes(ni, ncell);
@@ -887,6 +890,7 @@ int build_device_impl(mv_context* ctx, const double* d_xyz, const uint8_t* d_mas
     J.precision = o.precision;
     set_job_geometry(J, s);
     J.ext = C->ext;
+    J.outside = got[1];
     J.ppc_mean = (double)std::max<int64_t>(n, 1) / (double)ncell;
     J.volume = P<double>(W.volume);
     J.centroid = P<double>(W.centroid);
@@ -1093,7 +1097,10 @@ int build_batch_device_impl(mv_context* ctx, const double* d_xyz, const uint8_t*
     if (ntot >= INT32_MAX || ctot >= INT32_MAX) return MV_ERR_ARG;
     BatchGrid& g = bg[j];
     std::memset(&g, 0, sizeof(g));
-    for (int i = 0; i < 3; i++) g.G[i] = S[j].G[i], g.a[i] = S[j].anchor[i], g.inv[i] = S[j].ginv[i];
+    for (int i = 0; i < 3; i++) {
+      g.G[i] = S[j].G[i], g.a[i] = S[j].anchor[i], g.inv[i] = S[j].ginv[i];
+      g.top[i] = S[j].anchor[i] + S[j].width[i];
+    }
     g.dim = S[j].dim;
     g.cbase = cb[j];
     any_mask |= jb.has_mask != 0;
@@ -1147,7 +1154,7 @@ int build_batch_device_impl(mv_context* ctx, const double* d_xyz, const uint8_t*
   e |= ensure(ctx, W.b_cbase, 4 * (size_t)(nj + 1));
   e |= ensure(ctx, W.b_grid, sizeof(BatchGrid) * (size_t)nj);
   e |= ensure(ctx, W.b_ext_keys, 8 * 6 * (size_t)nj);
-  e |= ensure(ctx, W.b_ext, 8 * 6 * (size_t)nj);
+  e |= ensure(ctx, W.b_ext, 8 * EXT_WORDS * (size_t)nj);
   e |= ensure(ctx, W.b_fbase, 8 * (size_t)(nj + 1));
   e |= ensure(ctx, W.b_cbconn, 8 * (size_t)(nj + 1));
   if (e) return MV_ERR_OOM;
@@ -1218,7 +1225,7 @@ int build_batch_device_impl(mv_context* ctx, const double* d_xyz, const uint8_t*
       J.face_mode = o.face_mode;
       J.precision = o.precision;
       set_job_geometry(J, sj);
-      J.ext = P<double>(W.b_ext) + 6 * j;
+      J.ext = P<double>(W.b_ext) + EXT_WORDS * j;
       J.ppc_mean = (double)std::max<int64_t>(jobs[j].n, 1) / (double)(cb[j + 1] - cb[j] - 1);
       J.volume = P<double>(W.volume) + pb;
       J.centroid = P<double>(W.centroid) + 3 * pb;

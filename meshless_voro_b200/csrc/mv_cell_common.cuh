@@ -206,8 +206,6 @@ struct CellCount {
 #define WCNT(CC, slot, v) ((CC).c[slot] += (unsigned)(v))
 
 // ------------------------------------------------------------- neighbour shell --
-// First position in [a, b) whose dense-cell key is >= k (the keys of a dense cell are
-// sorted).
 // The generators of a dense cell, [cs, ce), searched by a whole warp, a key pair per lane:
 // lane l holds the key of every step-th generator, so that a search finds its 32nd of the
 // cell by shuffles and only the rest by dependent loads, the pair's two searches side by
@@ -526,6 +524,29 @@ __device__ __noinline__ ShellCount flush_call(const Job& J, ShellBuf<CMAX>& B, i
   return flush_segments<CMAX, BIG, true, CODE_ONLY>(J, B, lane, x, R2, lo2, nsegs, total, count, stop, big);
 }
 
+// The grid cells [*lo, *hi] of a query along axis i, [x - R, x + R] in cells, for a build with
+// generators outside the box.  Those are in the cells at its walls, whose generators so lie
+// as far beyond the wall as the generators' extent: the wall cells that the query reaches
+// join its range.
+__device__ __forceinline__ void reach_walls(const Job& J, int i, double x, double R, const double* ext, bool wrap,
+                                            int* lo, int* hi) {
+  const int G = J.G[i];
+  if (!wrap) {
+    *lo = min(*lo, G - 1), *hi = max(*hi, 0);
+    return;
+  }
+  const double over = fmax(ext[3 + i] - (J.ga[i] + J.gw[i]), 0.0), under = fmax(J.ga[i] - ext[i], 0.0);
+  const double first = floor((x - R - J.geps[i] - over - J.ga[i]) * J.ginv[i]);
+  const double last = floor((x + R + J.geps[i] + under - J.ga[i]) * J.ginv[i]);
+#pragma unroll 1
+  for (int m = 1; m >= -1; m--) {  // the wall cells of image m above, of image -m below
+    const int upper = (m + 1) * G - 1, lower = -m * G;
+    if (upper < *lo && (double)upper >= first) *lo = upper;
+    if (lower > *hi && (double)lower <= last) *hi = lower;
+  }
+  *lo = min(*lo, 2 * G - 1), *hi = max(*hi, -G);
+}
+
 // Gathers every stream element (generator, periodic image) with lo2 <= d2 < R*R into
 // B (unsorted) and returns how many there are (may exceed CMAX; once the count passes
 // stop the gather ends early and returns a count above stop).  With BIG and a slot,
@@ -545,7 +566,7 @@ __device__ __noinline__ ShellCount flush_call(const Job& J, ShellBuf<CMAX>& B, i
 // the one-level form, a third of the size, is faster unrolled (128^3 Poisson shells 7.6 ms,
 // rolled 8.2).  8.4 M generators, half of them in clumps: 843 -> 780 ms for the build, with
 // dense_search and the sparse runs of a deferred segment taken together.
-template <int CMAX, bool BIG, bool DENSE, bool CODE_ONLY>
+template <int CMAX, bool BIG, bool DENSE, bool CODE_ONLY, bool OUTSIDE>
 __device__ __noinline__ int gather_shell_impl(const Job& J, ShellBuf<CMAX>& B, int lane, D3 x, double R,
                                               double lo2, const double* ext, bool* exhausted,
                                               int stop, char* big) {
@@ -564,6 +585,7 @@ __device__ __noinline__ int gather_shell_impl(const Job& J, ShellBuf<CMAX>& B, i
     double fh = floor((xa[i] + R + J.geps[i] - J.ga[i]) * J.ginv[i]);
     lo[i] = fl < (double)umin ? umin : (int)fl;
     hi[i] = fh > (double)umax ? umax : (int)fh;
+    if (OUTSIDE) reach_walls(J, i, xa[i], R, ext, wrap, &lo[i], &hi[i]);
     if (lo[i] > umin || hi[i] < umax) all = false;
   }
   const double R2 = R * R;
@@ -746,7 +768,8 @@ __device__ __noinline__ int gather_shell_impl(const Job& J, ShellBuf<CMAX>& B, i
           int a = max(first, mx * Gx), b = min(last, mx * Gx + Gx - 1);
           if (a > b) continue;
           int c0 = a - mx * Gx, c1 = b - mx * Gx;
-          if (DENSE && __ldg(J.dprefix + rowbase + c1 + 1) > __ldg(J.dprefix + rowbase + c0)) {
+          if (DENSE && (!OUTSIDE || J.dprefix != nullptr) &&
+              __ldg(J.dprefix + rowbase + c1 + 1) > __ldg(J.dprefix + rowbase + c0)) {
             dfr[mx + 1] = c0 | (c1 << 16);
             continue;
           }
@@ -831,16 +854,22 @@ __device__ __noinline__ int gather_shell_impl(const Job& J, ShellBuf<CMAX>& B, i
 }
 
 // gather_shell_impl without the dense-cell code when the build has no dense cell (the
-// uniform-density case keeps its registers), with it otherwise.
+// uniform-density case keeps its registers), with it otherwise; a third form takes the
+// builds with generators outside the box, whose wider ranges of cells would cost the others
+// registers.  OUT: the build may have such generators, and ext tells.  Even the question costs
+// (128^3 Poisson shells 6.9 ms, with it 7.1, with the wider ranges in all forms 7.5), so that
+// a kernel of a single build whose host knows the answer is compiled without it.
 // With CODE_ONLY, B.tie holds the shift code alone (no load of the original index per
 // element); the caller completes it where the full order is needed.
-template <int CMAX, bool BIG = false, bool CODE_ONLY = false>
+template <int CMAX, bool OUT, bool BIG = false, bool CODE_ONLY = false>
 __device__ __forceinline__ int gather_shell(const Job& J, ShellBuf<CMAX>& B, int lane, D3 x, double R,
                                             double lo2, const double* ext, bool* exhausted, int stop,
                                             char* big = nullptr) {
+  if (OUT && ext[6] != 0.0)
+    return gather_shell_impl<CMAX, BIG, true, CODE_ONLY, true>(J, B, lane, x, R, lo2, ext, exhausted, stop, big);
   return J.dprefix != nullptr
-             ? gather_shell_impl<CMAX, BIG, true, CODE_ONLY>(J, B, lane, x, R, lo2, ext, exhausted, stop, big)
-             : gather_shell_impl<CMAX, BIG, false, CODE_ONLY>(J, B, lane, x, R, lo2, ext, exhausted, stop, big);
+             ? gather_shell_impl<CMAX, BIG, true, CODE_ONLY, false>(J, B, lane, x, R, lo2, ext, exhausted, stop, big)
+             : gather_shell_impl<CMAX, BIG, false, CODE_ONLY, false>(J, B, lane, x, R, lo2, ext, exhausted, stop, big);
 }
 
 // Bitonic sort of the shell [0, n) by (key, tie) ascending, carrying cpos; n <= CMAX.

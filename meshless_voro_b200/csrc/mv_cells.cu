@@ -172,7 +172,7 @@ __device__ __forceinline__ void setup_batch(const Job& J, CellSmem<T>& S, int la
   __syncwarp();
 }
 
-template <class T, int PREC>
+template <class T, int PREC, bool OUT>
 __device__ int build_cell(const Job& J, CellSmem<T>& S, int lane, int spos, const double* ext,
                           int* err_code, CellCount& cc) {
   using PIdx = typename T::PIdx;
@@ -220,7 +220,7 @@ __device__ int build_cell(const Job& J, CellSmem<T>& S, int lane, int spos, cons
     bool all;
     // what this shell may hold: the shared buffer, or a staging slot
     const int fits = big_fits<T::CMAX>(J);
-    int cnt = gather_shell<T::CMAX, true>(J, S.u.g.sh, lane, x, R, lo2, ext, &all, fits, big_slot(J));
+    int cnt = gather_shell<T::CMAX, OUT, true>(J, S.u.g.sh, lane, x, R, lo2, ext, &all, fits, big_slot(J));
     int shrink = 0;
     bool staged = false;
     for (;;) {
@@ -236,7 +236,7 @@ __device__ int build_cell(const Job& J, CellSmem<T>& S, int lane, int spos, cons
       const double rin3 = lo2 * sqrt(lo2);
       const double g = fmin(fmax(0.5 * (double)(J.big != nullptr ? fits : T::CMAX) / (double)cnt, 1e-3), 0.7);
       R = cbrt(rin3 + (R * R * R - rin3) * g);
-      cnt = gather_shell<T::CMAX, true>(J, S.u.g.sh, lane, x, R, lo2, ext, &all, fits, big_slot(J));
+      cnt = gather_shell<T::CMAX, OUT, true>(J, S.u.g.sh, lane, x, R, lo2, ext, &all, fits, big_slot(J));
       shrink++;
     }
     if (cnt > T::CMAX && !staged) return CELL_OVERFLOW;
@@ -467,14 +467,14 @@ __device__ int build_cell(const Job& J, CellSmem<T>& S, int lane, int spos, cons
   return res;
 }
 
-template <class T, int PREC, int WARPS, bool MULTI>
+template <class T, int PREC, int WARPS, bool MULTI, bool OUT>
 __global__ void __launch_bounds__(32 * WARPS, T::MINB)
     cells_kernel(const __grid_constant__ Job J0, const __grid_constant__ JobTable TB) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   CellSmem<T>& S = reinterpret_cast<CellSmem<T>*>(smem_raw)[warp];
-  __shared__ double ext_s[6];
-  if (threadIdx.x < 6) ext_s[threadIdx.x] = J0.ext[threadIdx.x];
+  __shared__ double ext_s[EXT_WORDS];
+  if (threadIdx.x < EXT_WORDS) ext_s[threadIdx.x] = J0.ext[threadIdx.x];
   if (lane < ST_COUNT) S.cnt[lane] = 0ull;
   __syncthreads();
   const int total = J0.order ? J0.n_order : J0.n;
@@ -505,7 +505,7 @@ __global__ void __launch_bounds__(32 * WARPS, T::MINB)
     CellCount cc;
 #pragma unroll
     for (int i = 0; i < ST_COUNT; i++) cc.c[i] = 0u;
-    const int res = build_cell<T, PREC>(J, S, lane, spos, ext, &err, cc);
+    const int res = build_cell<T, PREC, OUT>(J, S, lane, spos, ext, &err, cc);
     __syncwarp();
     if (res == CELL_DONE) cc.c[ST_CELLS]++;
     if (lane == 0) {
@@ -546,7 +546,7 @@ template <class T, int PREC, int WARPS>
 static int blocks_per_sm() {
   int nb = 0;
   const size_t smem = sizeof(CellSmem<T>) * WARPS;
-  auto k = cells_kernel<T, PREC, WARPS, false>;
+  auto k = cells_kernel<T, PREC, WARPS, false, false>;
   if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     return 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, 32 * WARPS, smem) != cudaSuccess) return 0;
@@ -556,7 +556,9 @@ static int blocks_per_sm() {
 template <class T, int PREC, int WARPS>
 static cudaError_t launch_tier(const Job& J, const JobTable& TB, int blocks, cudaStream_t st) {
   const size_t smem = sizeof(CellSmem<T>) * WARPS;
-  auto k = TB.jobs != nullptr ? cells_kernel<T, PREC, WARPS, true> : cells_kernel<T, PREC, WARPS, false>;
+  auto k = TB.jobs != nullptr ? cells_kernel<T, PREC, WARPS, true, true>
+                              : (J.outside ? cells_kernel<T, PREC, WARPS, false, true>
+                                           : cells_kernel<T, PREC, WARPS, false, false>);
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   k<<<blocks, 32 * WARPS, smem, st>>>(J, TB);

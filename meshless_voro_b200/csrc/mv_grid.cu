@@ -58,9 +58,26 @@ __global__ void prep_kernel(const double* __restrict__ xyz, int n, int dim, doub
   }
 }
 
-__global__ void ext_finish_kernel(const unsigned long long* ext_keys, double* ext) {
-  int i = threadIdx.x;
-  if (i < 6) ext[i] = ord_val(ext_keys[i]);
+// Word w of the extent that keys hold (EXT_WORDS); box: its lower and upper corner.
+__device__ __forceinline__ double ext_word(const unsigned long long* keys, int w, int dim, const double* a,
+                                           const double* top) {
+  if (w < 6) return ord_val(keys[w]);
+  bool outside = false;
+  for (int i = 0; i < dim; i++) outside |= ord_val(keys[i]) < a[i] || ord_val(keys[3 + i]) > top[i];
+  return outside ? 1.0 : 0.0;
+}
+
+struct Corners {
+  double a[3], top[3];
+};
+
+__global__ void ext_finish_kernel(const unsigned long long* ext_keys, double* ext, int dim, Corners box,
+                                  int32_t* outside /* null: not wanted */) {
+  const int w = threadIdx.x;
+  if (w >= EXT_WORDS) return;
+  const double v = ext_word(ext_keys, w, dim, box.a, box.top);
+  ext[w] = v;
+  if (w == 6 && outside != nullptr) *outside = v != 0.0;
 }
 
 struct GridParams {
@@ -462,9 +479,10 @@ __global__ void batch_prep_kernel(const double* __restrict__ xyz, int n, const i
   }
 }
 
-__global__ void batch_ext_finish_kernel(const unsigned long long* ext_keys, double* ext, int nj) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < 6 * nj) ext[i] = ord_val(ext_keys[i]);
+__global__ void batch_ext_finish_kernel(const unsigned long long* ext_keys, double* ext,
+                                        const BatchGrid* __restrict__ bg, int nj) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, j = i / EXT_WORDS;
+  if (j < nj) ext[i] = ext_word(ext_keys + 6 * j, i % EXT_WORDS, bg[j].dim, bg[j].a, bg[j].top);
 }
 
 // grid cell (batch-wide index) of each generator, and the cell counts
@@ -580,10 +598,12 @@ __global__ void batch_local_conn_kernel(int64_t* __restrict__ conn_off,
 // ---------------------------------------------------------------- launchers --
 static inline int nblk(int64_t n, int t) { return (int)((n + t - 1) / t); }
 
-void launch_prep(const double* xyz, int n, int dim, double* gen, unsigned long long* ext_keys,
-                 double* ext, int* bad, cudaStream_t st) {
+void launch_prep(const double* xyz, int n, int dim, const double anchor[3], const double width[3], double* gen,
+                 unsigned long long* ext_keys, double* ext, int32_t* outside, int* bad, cudaStream_t st) {
+  Corners box;
+  for (int i = 0; i < 3; i++) box.a[i] = anchor[i], box.top[i] = anchor[i] + width[i];
   if (n > 0) prep_kernel<<<nblk(n, 256), 256, 0, st>>>(xyz, n, dim, gen, ext_keys, bad);
-  ext_finish_kernel<<<1, 32, 0, st>>>(ext_keys, ext);
+  ext_finish_kernel<<<1, 32, 0, st>>>(ext_keys, ext, dim, box, outside);
 }
 
 void launch_grid(const double* gen, int n, const int G[3], const double a[3], const double inv[3],
@@ -722,7 +742,7 @@ int launch_batch_grid(const double* xyz, int n, const int32_t* pos, const int32_
                       int32_t* dflag, int32_t* dprefix, long long* scan_tmp, cudaStream_t st) {
   batch_ext_init_kernel<<<nblk(6 * (int64_t)nj, 256), 256, 0, st>>>(ext_keys, nj);
   if (n > 0) batch_prep_kernel<<<nblk(n, 256), 256, 0, st>>>(xyz, n, pos, nj, bg, gen, ext_keys, bad);
-  batch_ext_finish_kernel<<<nblk(6 * (int64_t)nj, 256), 256, 0, st>>>(ext_keys, ext, nj);
+  batch_ext_finish_kernel<<<nblk(EXT_WORDS * (int64_t)nj, 256), 256, 0, st>>>(ext_keys, ext, bg, nj);
   if (n > 0) batch_cell_index_kernel<<<nblk(n, 256), 256, 0, st>>>(gen, n, pos, nj, bg, cid, count);
   const int launches = 5 + scan_i32_to_i32(count, ncell, start, scan_tmp, st);
   dense_flag_kernel<<<nblk(ncell, 256), 256, 0, st>>>(count, ncell, dflag);

@@ -24,12 +24,16 @@ enum StatSlot {
 enum { STATUS_CODE = 0, STATUS_CELL = 1, STATUS_FACE_OVERFLOW = 2, STATUS_REC_OVERFLOW = 3,
        STATUS_WORDS = 4 };
 
+// The generators' extent: minimum of x, y, z, maximum of x, y, z, and 1 where a generator
+// lies outside the box (else 0).
+constexpr int EXT_WORDS = 7;
+
 // Device counters of one build (one allocation, cleared before each build).
 struct DevCounters {
   unsigned long long face_counter;
   unsigned long long stats[ST_COUNT];
   unsigned long long ext_keys[6];
-  double ext[6];
+  double ext[EXT_WORDS];
   int32_t status[STATUS_WORDS];
   unsigned int work[4];       // work queues of the capacity tiers
   unsigned int ovf_count[4];  // overflow lists of the capacity tiers
@@ -69,7 +73,8 @@ struct Job {
   double gw[3];             // normalised simulation width (period of the images)
   double gh[3];             // cell size
   double ginv[3];           // 1 / cell size
-  const double* ext;        // device [6]: min x,y,z, max x,y,z of the generators
+  const double* ext;        // device [EXT_WORDS]
+  int32_t outside;          // 0: the host knows that ext[6] is 0
   double geps[3];           // cell-box inflation against rounding of the cell index
   double R0;                // first neighbour-shell radius
   // second level in dense cells (all nullptr when no cell is dense): the generators of a
@@ -168,7 +173,7 @@ struct StageJob {
 struct BatchGrid {
   int G[3];
   int dim;
-  double a[3], inv[3];
+  double a[3], top[3], inv[3];  // the box's lower and upper corner, 1 / cell size
   int32_t cbase;  // first batch-wide grid cell of the tessellation
   int32_t pad;
 };

@@ -34,8 +34,8 @@ namespace mv {
 cudaError_t launch_cells(const Job& J, bool large, int blocks, cudaStream_t st, const JobTable& TB);
 int cells_blocks_per_sm_fast(int precision);
 int cells_blocks_per_sm_large(int precision);
-void launch_prep(const double* xyz, int n, int dim, double* gen, unsigned long long* ext_keys,
-                 double* ext, int* bad, cudaStream_t st);
+void launch_prep(const double* xyz, int n, int dim, const double anchor[3], const double width[3], double* gen,
+                 unsigned long long* ext_keys, double* ext, int32_t* outside, int* bad, cudaStream_t st);
 void launch_grid(const double* gen, int n, const int G[3], const double a[3], const double inv[3],
                  int32_t* cid, int32_t* count, int32_t* start, int32_t* fill, double* sx, double* sy,
                  double* sz, int32_t* sid, long long* scan_tmp, cudaStream_t st);
@@ -194,7 +194,8 @@ extern "C" int mv_voronoi_build_noalloc(const double* d_generators, const uint8_
   NA_CUDA(cudaMemsetAsync(B + O_CCOUNT, 0, 4 * (ncell + 1), st));
   NA_CUDA(cudaMemsetAsync(B + O_CFILL, 0, 4 * (ncell + 1), st));
 
-  launch_prep(d_generators, ni, s.dim, at<double>(B, O_GEN), C->ext_keys, C->ext, &C->bad_input, st);
+  launch_prep(d_generators, ni, s.dim, s.anchor, s.width, at<double>(B, O_GEN), C->ext_keys, C->ext, nullptr,
+              &C->bad_input, st);
   launch_grid(at<double>(B, O_GEN), ni, s.G, s.anchor, s.ginv, at<int32_t>(B, O_CID),
               at<int32_t>(B, O_CCOUNT), at<int32_t>(B, O_CSTART), at<int32_t>(B, O_CFILL),
               at<double>(B, O_SX), at<double>(B, O_SY), at<double>(B, O_SZ), at<int32_t>(B, O_SID),
@@ -225,6 +226,7 @@ extern "C" int mv_voronoi_build_noalloc(const double* d_generators, const uint8_
     J.iloc_inv[i] = s.iloc_inv[i];
   }
   J.ext = C->ext;
+  J.outside = 1;  // not asked: reading it back would be one more wait of the host
   J.R0 = s.R0;
   for (int c = 0; c < 27; c++) {
     const int m[3] = {c % 3 - 1, (c / 3) % 3 - 1, c / 9 - 1};

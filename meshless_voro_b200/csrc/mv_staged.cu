@@ -140,15 +140,15 @@ __device__ __forceinline__ bool sort_and_write(const Job& J, const ShellBuf<SHEL
   return __shfl_sync(FULL, first, 0) == (uint32_t)spos * 27u + 13u;
 }
 
-template <int WARPS, bool MULTI>
+template <int WARPS, bool MULTI, bool OUT>
 __global__ void __launch_bounds__(32 * WARPS, MV_SHELL_MINB)
     shell_kernel(const __grid_constant__ Job J0, const __grid_constant__ StageJob SJ,
                  const __grid_constant__ JobTable TB) {
   __shared__ ShellBuf<SHELL_CMAX> bufs[WARPS];
-  __shared__ double ext_s[6];
+  __shared__ double ext_s[EXT_WORDS];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   ShellBuf<SHELL_CMAX>& B = bufs[warp];
-  if (threadIdx.x < 6) ext_s[threadIdx.x] = J0.ext[threadIdx.x];
+  if (threadIdx.x < EXT_WORDS) ext_s[threadIdx.x] = J0.ext[threadIdx.x];
   __syncthreads();
   for (;;) {
     int item = 0;
@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(32 * WARPS, MV_SHELL_MINB)
     const D3 x = load_gen(J, self);
     bool all = false;
     double R = first_radius(J, x, lane);
-    int cnt = gather_shell<SHELL_CMAX, false, true>(J, B, lane, x, R, 0.0, ext, &all, 32 * SHELL_CMAX);
+    int cnt = gather_shell<SHELL_CMAX, OUT, false, true>(J, B, lane, x, R, 0.0, ext, &all, 32 * SHELL_CMAX);
     // the density estimate behind R is rough where the density varies: a shell that
     // overflows the list is pulled in, one far below a uniform region's ~92 candidates
     // (too small to close most cells) is widened, a few times at most
@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(32 * WARPS, MV_SHELL_MINB)
       else
         break;
       R *= f;
-      cnt = gather_shell<SHELL_CMAX, false, true>(J, B, lane, x, R, 0.0, ext, &all, 32 * SHELL_CMAX);
+      cnt = gather_shell<SHELL_CMAX, OUT, false, true>(J, B, lane, x, R, 0.0, ext, &all, 32 * SHELL_CMAX);
     }
     if (cnt > SHELL_CMAX || cnt == 0) {
       if (lane == 0) SJ.info[item] = -1;
@@ -256,15 +256,15 @@ __device__ __noinline__ bool sort_shell_key32(ShellBuf<CMAX>& B, int lane, int n
   return !__any_sync(FULL, dup);
 }
 
-template <int WARPS, bool MULTI>
+template <int WARPS, bool MULTI, bool OUT>
 __global__ void __launch_bounds__(32 * WARPS, 3)
     shell_wide_kernel(const __grid_constant__ Job J0, const __grid_constant__ StageJob SJ,
                       const __grid_constant__ JobTable TB) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ double ext_s[6];
+  __shared__ double ext_s[EXT_WORDS];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   ShellBuf<WIDE_CMAX>& B = reinterpret_cast<ShellBuf<WIDE_CMAX>*>(smem_raw)[warp];
-  if (threadIdx.x < 6) ext_s[threadIdx.x] = J0.ext[threadIdx.x];
+  if (threadIdx.x < EXT_WORDS) ext_s[threadIdx.x] = J0.ext[threadIdx.x];
   __syncthreads();
   for (;;) {
     int item = 0;
@@ -288,7 +288,7 @@ __global__ void __launch_bounds__(32 * WARPS, 3)
     const int least = even ? 128 : 384;  // widened below this many candidates
     const double aim = even ? 256.0 : 768.0;
     double R = (even ? 1.4 : 2.0) * first_radius(J, x, lane);
-    int cnt = gather_shell<WIDE_CMAX>(J, B, lane, x, R, 0.0, ext, &all, 4 * WIDE_CMAX);
+    int cnt = gather_shell<WIDE_CMAX, OUT>(J, B, lane, x, R, 0.0, ext, &all, 4 * WIDE_CMAX);
     for (int it = 0; it < 6; it++) {
       double f;
       if (cnt > WIDE_CMAX)
@@ -298,7 +298,7 @@ __global__ void __launch_bounds__(32 * WARPS, 3)
       else
         break;
       R *= f;
-      cnt = gather_shell<WIDE_CMAX>(J, B, lane, x, R, 0.0, ext, &all, 4 * WIDE_CMAX);
+      cnt = gather_shell<WIDE_CMAX, OUT>(J, B, lane, x, R, 0.0, ext, &all, 4 * WIDE_CMAX);
     }
     if (cnt > WIDE_CMAX || cnt == 0) {
       if (lane == 0) SJ.info[item] = -1;
@@ -314,7 +314,7 @@ __global__ void __launch_bounds__(32 * WARPS, 3)
       first = B.tie[(uint32_t)B.key[0]];
     } else {
       // equal keys: the same shell again (the gather is deterministic), fully sorted
-      cnt = gather_shell<WIDE_CMAX>(J, B, lane, x, R, 0.0, ext, &all, 4 * WIDE_CMAX);
+      cnt = gather_shell<WIDE_CMAX, OUT>(J, B, lane, x, R, 0.0, ext, &all, 4 * WIDE_CMAX);
       sort_shell<WIDE_CMAX>(B, lane, cnt);
       for (int i = lane; i < cnt; i += 32) out[i] = (uint32_t)B.cpos[i] * 27u + B.tie[i] % 27u;
       first = B.tie[0];
@@ -381,8 +381,8 @@ static int occupancy(K k, int threads, size_t smem) {
 }
 
 int stage_blocks_per_sm(int kernel) {
-  if (kernel == 0) return occupancy(shell_kernel<SHELL_WARPS, false>, 32 * SHELL_WARPS, 0);
-  if (kernel == 3) return occupancy(shell_wide_kernel<WIDE_WARPS, false>, 32 * WIDE_WARPS, WIDE_SMEM);
+  if (kernel == 0) return occupancy(shell_kernel<SHELL_WARPS, false, false>, 32 * SHELL_WARPS, 0);
+  if (kernel == 3) return occupancy(shell_wide_kernel<WIDE_WARPS, false, false>, 32 * WIDE_WARPS, WIDE_SMEM);
   return occupancy(integrate_kernel<TierClip, INT_WARPS, false>, 32 * INT_WARPS, 0);
 }
 
@@ -403,13 +403,13 @@ int stage_wide_stride() { return WIDE_CMAX; }
 
 int64_t stage_record_words(int np, int nv) { return rec_words(np, nv); }
 
-template <bool MULTI>
+template <bool MULTI, bool OUT>
 static cudaError_t launch_stage_t(int kernel, const Job& J, const StageJob& SJ, const JobTable& TB,
                                   int blocks, cudaStream_t st) {
   if (kernel == 0) {
-    shell_kernel<SHELL_WARPS, MULTI><<<blocks, 32 * SHELL_WARPS, 0, st>>>(J, SJ, TB);
+    shell_kernel<SHELL_WARPS, MULTI, OUT><<<blocks, 32 * SHELL_WARPS, 0, st>>>(J, SJ, TB);
   } else if (kernel == 3) {
-    auto k = shell_wide_kernel<WIDE_WARPS, MULTI>;
+    auto k = shell_wide_kernel<WIDE_WARPS, MULTI, OUT>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WIDE_SMEM);
     if (e != cudaSuccess) return e;
     k<<<blocks, 32 * WIDE_WARPS, WIDE_SMEM, st>>>(J, SJ, TB);
@@ -424,8 +424,9 @@ static cudaError_t launch_stage_t(int kernel, const Job& J, const StageJob& SJ, 
 cudaError_t launch_stage(int kernel, const Job& J, const StageJob& SJ, const JobTable& TB, int blocks,
                          cudaStream_t st) {
   if (blocks < 1) blocks = 1;
-  return TB.jobs != nullptr ? launch_stage_t<true>(kernel, J, SJ, TB, blocks, st)
-                            : launch_stage_t<false>(kernel, J, SJ, TB, blocks, st);
+  if (TB.jobs != nullptr) return launch_stage_t<true, true>(kernel, J, SJ, TB, blocks, st);
+  return J.outside ? launch_stage_t<false, true>(kernel, J, SJ, TB, blocks, st)
+                   : launch_stage_t<false, false>(kernel, J, SJ, TB, blocks, st);
 }
 
 }  // namespace mv
