@@ -296,6 +296,13 @@ __device__ __forceinline__ double first_radius(const Job& J, D3 x, int lane) {
   if (!(ratio > 1.0f)) return J.R0;
   return J.R0 * (double)exp2f(log2f(ratio) * (-1.0f / dim));
 }
+// the same, out of the caller's code
+static __device__ __noinline__ double first_radius_dense(const Job& J, D3 x, int lane) {
+  return first_radius(J, x, lane);
+}
+__device__ __forceinline__ double first_radius_call(const Job& J, D3 x, int lane) {
+  return J.fkey == nullptr ? J.R0 : first_radius_dense(J, x, lane);
+}
 
 template <int CMAX>
 struct ShellBuf {
