@@ -43,7 +43,7 @@ cudaError_t launch_stage(int kernel, const Job& J, const StageJob& SJ, const Job
                          cudaStream_t st);
 int stage_blocks_per_sm(int kernel);
 // mv_clip.cu
-cudaError_t launch_clip(const Job& J, const StageJob& SJ, const JobTable& TB, bool wide, int resident,
+cudaError_t launch_clip(const Job& J, const StageJob& SJ, const JobTable& TB, bool wide, bool uneven, int resident,
                         cudaStream_t st);
 int clip_cells_per_block();
 int clip_blocks_per_sm(int precision, bool wide);
@@ -362,8 +362,8 @@ cudaError_t run_stage_kernel(const mv_context* ctx, int kernel, const Job& J, co
     // generators: 0.54 ms with the first tier, 0.41 ms with the wide one)
     const int wide = ctx->sm_count * std::max(1, ctx->bps_stage[4][pi]);
     if (kernel == 4 || SJ.nitems <= (int64_t)wide * clip_cells_per_block())
-      return launch_clip(J, SJ, TB, true, wide, st);
-    return launch_clip(J, SJ, TB, false, resident, st);
+      return launch_clip(J, SJ, TB, true, kernel == 4 && TB.jobs == nullptr && J.fkey != nullptr, wide, st);
+    return launch_clip(J, SJ, TB, false, false, resident, st);
   }
   return launch_stage(kernel, J, SJ, TB, std::max(1, std::min(resident, (SJ.nitems + 3) / 4)), st);
 }
