@@ -31,9 +31,6 @@
 
 namespace mv {
 
-#ifndef MV_CLIP_G
-#define MV_CLIP_G 8
-#endif
 #ifndef MV_CLIP_WARPS
 #define MV_CLIP_WARPS 2
 #endif
@@ -49,27 +46,27 @@ namespace mv {
 
 // Capacities of one cell: PMAX planes and VMAX vertices; a cell that outgrows them goes
 // on to the next round.
-template <int G_, int VMAX_, int PMAX_, int WARPS_, int MINB_>
+template <int VMAX_, int PMAX_, int WARPS_, int MINB_>
 struct ClipTier {
-  static constexpr int G = G_;          // lanes per cell
-  static constexpr int NG = 32 / G_;    // cells per warp
+  static constexpr int G = 8;           // lanes per cell
+  static constexpr int NG = 32 / G;     // cells per warp
   static constexpr int VMAX = VMAX_;
   static constexpr int PMAX = PMAX_;
   static constexpr int WARPS = WARPS_;
   static constexpr int MINB = MINB_;    // resident blocks per SM the registers are sized for
-  static constexpr int WIN = 2 * G_;    // candidates in the window (refilled G at a time)
+  static constexpr int WIN = 2 * G;     // candidates in the window (refilled G at a time)
   static constexpr int RMAX = 32;       // removed vertices, ring edges
-  static constexpr int NC = VMAX_ / G_; // vertices per lane
+  static constexpr int NC = VMAX_ / G;  // vertices per lane
   // bytes per plane: words, and the successor of a node outside the ring.  No plane has the
   // number PMAX, so its byte is free: it stays NONE, and a walk that leaves a broken ring
   // goes on inside the table
   static constexpr int PW = (PMAX_ + 4) / 4;
   static constexpr unsigned NONE = PMAX_;
   static constexpr uint32_t NONE4 = 0x01010101u * NONE;
-  static_assert(G_ == 8 && VMAX_ % (2 * G_) == 0 && VMAX_ <= 64 && PMAX_ < 255, "tier");
+  static_assert(VMAX_ % (2 * G) == 0 && VMAX_ <= 64 && PMAX_ < 255, "tier");
 };
-using ClipFirst = ClipTier<MV_CLIP_G, MV_CLIP_VMAX, MV_CLIP_PMAX, MV_CLIP_WARPS, MV_CLIP_MINB>;
-using ClipWide = ClipTier<MV_CLIP_G, 64, 64, MV_CLIP_WARPS, 6>;
+using ClipFirst = ClipTier<MV_CLIP_VMAX, MV_CLIP_PMAX, MV_CLIP_WARPS, MV_CLIP_MINB>;
+using ClipWide = ClipTier<64, 64, MV_CLIP_WARPS, 6>;
 
 __device__ __forceinline__ uint32_t pack_dual(int i, int j, int k) {
   return (uint32_t)i | ((uint32_t)j << 8) | ((uint32_t)k << 16);
@@ -330,9 +327,6 @@ __device__ __forceinline__ void fill_window(const Job& J, SM& S, const uint32_t*
   }
 }
 
-__device__ __forceinline__ int low_bit(unsigned m) { return __ffs((int)m) - 1; }
-__device__ __forceinline__ int low_bit(unsigned long long m) { return __ffsll((long long)m) - 1; }
-
 // The swap-remove loop (convex_cell.rs:365-390) of the r removed vertices, one per lane,
 // with rm their positions and kr the kept ones in bit-reversed order: removed vertex j at
 // position p is replaced by the j-th kept vertex from the end (position q) when
@@ -460,7 +454,7 @@ __device__ __noinline__ int ring_start(uint32_t du, uint32_t M, uint32_t N, int 
 template <class T, class SM>
 __device__ __noinline__ unsigned ring_wide(SM& S, int gl, int gbase, bool on, int r) {
   constexpr int G = T::G;
-  constexpr unsigned GM = G == 32 ? FULL : ((1u << G) - 1u);
+  constexpr unsigned GM = (1u << G) - 1u;
   uint8_t* const rptr = reinterpret_cast<uint8_t*>(S.ring);
   if (on)
 #pragma unroll 1
@@ -589,7 +583,7 @@ __global__ void __launch_bounds__(32 * T::WARPS, T::MINB)
                 const __grid_constant__ JobTable TB) {
   constexpr int G = T::G, NC = T::NC, WIN = T::WIN;
   constexpr bool FILT = PREC == MV_PRECISION_FILTERED;
-  constexpr unsigned GM = G == 32 ? FULL : ((1u << G) - 1u);
+  constexpr unsigned GM = (1u << G) - 1u;
   using Cell = typename CellOf<T, PREC>::type;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
